@@ -4,6 +4,7 @@
 #include "gg_corrector.cuh"
 #include "gg_kernels.cuh"
 #include "gg_launch.cuh"
+#include "gg_redist.cuh"
 #include "gg_warp.cuh"
 
 namespace gg {
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(128) k_corrector_big(NetConst C, NetState* S) 
     }
 }
 
-// persistent grid of the large-box kernels: one CTA per SM
+// SMs of the device, the unit of the persistent grids
 int g_big_grid = 148;
 // highest stream priority of the device (numerically lowest)
 int g_high_priority = 0;
@@ -742,11 +743,30 @@ cudaError_t batched_resample(const NetConst& C, NetState* dS, double h_old, doub
     return cudaGetLastError();
 }
 
+// The large-box bin: a persistent grid walks the work queue (largest boxes
+// first) and stops at the first existing grain at or below C.big_edge, where
+// k_redistance's begin.
+__global__ void __launch_bounds__(RedistLarge<float>::kThreads, RedistLarge<float>::kPerSm)
+    k_redistance_big(NetConst C, NetState* S) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    if (!S->order) return;
+    for (int slot = blockIdx.x; slot < C.N; slot += gridDim.x) {
+        const int g = S->order[slot];
+        // a grain that vanished in this step's level set keeps its place in
+        // the queue; existing grains are in descending box edge
+        if (C.state[g] != G_EXISTS || halted(S)) continue;
+        if (box_w(S->box_cur[g]) <= C.big_edge) return;
+        redistance_grain<float, true>(C, S, g, s_raw);
+        __syncthreads();  // the next grain reuses the shared buffers
+    }
+}
+
 cudaError_t batched_prepare(int tmax) {
     cudaError_t e = cudaFuncSetAttribute(k_conv_sep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)conv_sep_smem(tmax, kConvSmemEdgeMax));
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_redistance_big, cudaFuncAttributeMaxDynamicSharedMemorySize, kRedistBigSmemBytes);
+    e = cudaFuncSetAttribute(k_redistance_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)redist_smem<float, true>());
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
@@ -758,12 +778,31 @@ cudaError_t batched_prepare(int tmax) {
     return cudaSuccess;
 }
 
-// The redistancing stage: the large-box bin, then the 64-thread kernel for
-// the rest.
+// The large-box bin of the redistancing, at the device's highest priority
+// (beside the main kernel its CTAs are placed first).
+void launch_redistance_big(const NetConst& C, NetState* dS, cudaStream_t s) {
+    using L = RedistLarge<float>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C.N < L::kPerSm * g_big_grid ? C.N : L::kPerSm * g_big_grid);
+    cfg.blockDim = dim3(L::kThreads);
+    cfg.dynamicSmemBytes = redist_smem<float, true>();
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributePriority;
+    attr[0].val.priority = g_high_priority;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_redistance_big, C, dS);
+}
+
+void launch_redistance_main(const NetConst& C, NetState* dS, cudaStream_t s) {
+    k_redistance<float, false><<<C.N, kRedistThreads, redist_smem<float, false>(), s>>>(C, dS);
+}
+
+// Both on one stream (the graph runs them on two).
 void launch_redistance(const NetConst& C, NetState* dS, cudaStream_t s) {
-    const int grid = C.N < g_big_grid ? C.N : g_big_grid;
-    k_redistance_big<<<grid, kRedistBigThreads, kRedistBigSmemBytes, s>>>(C, dS);
-    k_redistance_s<float><<<C.N, kRedistThreads, kRedistSmemBytes, s>>>(C, dS);
+    launch_redistance_big(C, dS, s);
+    launch_redistance_main(C, dS, s);
 }
 
 cudaError_t batched_init(const NetConst& C, NetState* dS, const int32_t* d_ids, cudaStream_t s) {
@@ -848,8 +887,8 @@ cudaError_t batched_stages(const NetConst& C, NetState* dS, int stages, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, cudaStream_t s2, cudaEvent_t* ev,
-                               const LaunchCfg& cfg) {
+cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, cudaStream_t s2, cudaStream_t s3,
+                               cudaEvent_t* ev, const LaunchCfg& cfg) {
     if (C.N <= 0) return cudaSuccess;
     const int wblocks = (C.N + kGrainsPerBlock - 1) / kGrainsPerBlock;
     cudaError_t e;
@@ -873,12 +912,16 @@ cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, 
     // volume / energy / neighbours (contours, lists) and the next step's
     // sectors beside redistancing (fields)
     if ((e = cudaEventRecord(ev[2], s)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(s3, ev[2], 0)) != cudaSuccess) return e;
+    launch_redistance_big(C, dS, s3);
+    if ((e = cudaEventRecord(ev[5], s3)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s2, ev[2], 0)) != cudaSuccess) return e;
     k_neighbours_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s2>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo));
     k_sectors<true><<<C.N, 32, 0, s2>>>(C, dS);  // the next step's sectors
     if ((e = cudaEventRecord(ev[3], s2)) != cudaSuccess) return e;
-    launch_redistance(C, dS, s);
+    launch_redistance_main(C, dS, s);
     if ((e = cudaStreamWaitEvent(s, ev[3], 0)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(s, ev[5], 0)) != cudaSuccess) return e;
     k_finalize<<<1, 1024, 0, s>>>(C, dS, 1);
     k_order<<<1, 1024, 0, s>>>(C, dS);  // the next step's work queue, from its boxes
     return cudaGetLastError();

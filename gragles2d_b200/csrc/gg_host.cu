@@ -123,8 +123,8 @@ struct gg_ctx {
     int32_t graph_kernels = 0;     // kernel nodes of the captured step graph
     int64_t kernel_launches = 0;   // graph_kernels per replay, summed
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaStream_t stream2 = nullptr;  // second branch of the captured batched step
-    cudaEvent_t fork[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    cudaStream_t stream2 = nullptr, stream3 = nullptr;  // further branches of the captured batched step
+    cudaEvent_t fork[kStepForks] = {};
     double last_ms = 0;
 
     ~gg_ctx() {
@@ -141,6 +141,7 @@ struct gg_ctx {
         for (cudaEvent_t e : fork)
             if (e) cudaEventDestroy(e);
         if (stream2) cudaStreamDestroy(stream2);
+        if (stream3) cudaStreamDestroy(stream3);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -830,7 +831,8 @@ int gg_create(const gg_params* p, int device, gg_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking);
-    for (int k = 0; k < 5 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&c->fork[k], cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking);
+    for (int k = 0; k < kStepForks && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&c->fork[k], cudaEventDisableTiming);
     if (e != cudaSuccess) {
         c->err = std::string("stream/event: ") + cudaGetErrorString(e);
         *out = c;
@@ -1274,7 +1276,7 @@ int gg_distance_initialisation(gg_ctx* c) {
     C.nbmax = 48;
     C.jmax = 48;
     C.tmax = tmax;
-    C.big_edge = 128;
+    C.big_edge = 64;
     C.conv_smem_edge = 64;
     C.isotropic = P.is_isotropic_network ? 1 : 0;
     C.use_mobility_model = P.use_mobility_model;
@@ -1478,7 +1480,7 @@ int gg_distance_initialisation(gg_ctx* c) {
     S.cont_used = cc;
     GG_CUDA(c, h2d(c->dS, &S, sizeof(NetState)));
 
-    if (!plain) GG_CUDA(c, batched_prepare(tmax));
+    GG_CUDA(c, plain ? plain_prepare() : batched_prepare(tmax));
     if (poly) {
         // the loaded polygon is the grain's contour until the first level-set
         // stage (energy and mobility 0, no junctions); its area is
@@ -1676,7 +1678,7 @@ int gg_autotune(gg_ctx* c, int32_t loop, int32_t steps_per_candidate, gg_tuning*
         *knob = chosen;
         return GG_OK;
     };
-    if ((rc = tune(&c->C.big_edge, {64, 96, 128, 192, 1 << 20})) != GG_OK) return rc;
+    if ((rc = tune(&c->C.big_edge, {48, 56, 64})) != GG_OK) return rc;
     if ((rc = tune(&c->cfg.compare_threads, {128, 256})) != GG_OK) return rc;  // k_compare: at most 256
     if ((rc = tune(&c->C.conv_smem_edge, {48, 64, 96, 128})) != GG_OK) return rc;
     if (c->graph) {
@@ -1720,7 +1722,8 @@ int gg_step(gg_ctx* c, int32_t loop, int32_t nsteps) {
         if (!c->graph) {
             cudaGraph_t gr;
             GG_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = batched_step_graph(c->C, c->dS, c->stream, c->stream2, c->fork, c->cfg);
+            cudaError_t e = batched_step_graph(c->C, c->dS, c->stream, c->stream2, c->stream3, c->fork,
+                                               c->cfg);
             cudaError_t e2 = cudaStreamEndCapture(c->stream, &gr);
             if (e != cudaSuccess) return cuda_fail(c, e, "capture");
             if (e2 != cudaSuccess) return cuda_fail(c, e2, "end capture");

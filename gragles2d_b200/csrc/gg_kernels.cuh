@@ -675,96 +675,6 @@ __global__ void k_neighbours(NetConst C, NetState* S) {
     C.volume[g] = newVolume;
 }
 
-// ---------------------------------------------------------------------------
-// LSbox::executeRedistancing (src/box.cpp:1259-1399): one CTA per grain;
-// compared field (arena A, box_cur) -> phi_{t+1} (arena B, box_new).
-// y sweeps run one thread per column, x sweeps one thread per row.
-// ---------------------------------------------------------------------------
-template <typename R>
-__device__ void redistance_grain(const R* __restrict__ in, const Box bi, R* __restrict__ out, const Box bo, R h,
-                                 R delta) {
-    const int wi = box_w(bi), wo = box_w(bo);
-    const int64_t ao = box_area(bo);
-    for (int64_t p = threadIdx.x; p < ao; p += blockDim.x) out[p] = (R)-1.0;
-    __syncthreads();
-    const int ixmin = (bi.x0 < bo.x0) ? bo.x0 : bi.x0;
-    const int iymin = (bi.y0 < bo.y0) ? bo.y0 : bi.y0;
-    const int ixmax = (bi.x1 < bo.x1) ? bi.x1 : bo.x1;
-    const int iymax = (bi.y1 < bo.y1) ? bi.y1 : bo.y1;
-#define GG_IN(i, j) in[(int64_t)((i) - bi.y0) * wi + ((j) - bi.x0)]
-#define GG_OUT(i, j) out[(int64_t)((i) - bo.y0) * wo + ((j) - bo.x0)]
-    for (int j = ixmin + (int)threadIdx.x; j < bo.x1; j += blockDim.x) {
-        for (int i = iymin; i < bo.y1 - 1; i++) {  // y forward
-            R cand;
-            if (j < ixmax && i < iymax - 1) {
-                const R a = GG_IN(i, j), c = GG_IN(i + 1, j);
-                if (a * c <= (R)0.0) {
-                    const R slope = (c - a) / h;
-                    const R dz = -a / slope;
-                    if (fabs(GG_OUT(i, j)) > fabs(dz)) GG_OUT(i, j) = -dz * (R)sgn(slope);
-                }
-                cand = GG_OUT(i, j) + ((R)sgn(c) * h);
-            } else {
-                cand = GG_OUT(i, j) + ((R)sgn(GG_OUT(i + 1, j)) * h);
-            }
-            if (fabs(cand) < fabs(GG_OUT(i + 1, j))) GG_OUT(i + 1, j) = cand;
-        }
-        for (int i = iymax - 1; i > bo.y0; i--) {  // y backward
-            R cand;
-            if (j < ixmax && i > iymin)
-                cand = GG_OUT(i, j) + ((R)sgn(GG_IN(i - 1, j)) * h);
-            else
-                cand = GG_OUT(i, j) + ((R)sgn(GG_OUT(i - 1, j)) * h);
-            if (fabs(cand) < fabs(GG_OUT(i - 1, j))) GG_OUT(i - 1, j) = cand;
-        }
-    }
-    __syncthreads();
-    for (int i = iymin + (int)threadIdx.x; i < bo.y1; i += blockDim.x) {
-        for (int j = ixmin; j < bo.x1 - 1; j++) {  // x forward
-            R cand;
-            if (j < ixmax - 1 && i < iymax) {
-                const R a = GG_IN(i, j), c = GG_IN(i, j + 1);
-                if (a * c <= (R)0.0) {
-                    const R slope = (c - a) / h;
-                    const R dz = -a / slope;
-                    if (fabs(GG_OUT(i, j)) > fabs(dz)) GG_OUT(i, j) = -dz * (R)sgn(slope);
-                }
-                cand = GG_OUT(i, j) + ((R)sgn(c) * h);
-            } else {
-                cand = GG_OUT(i, j) + ((R)sgn(GG_OUT(i, j + 1)) * h);
-            }
-            if (fabs(cand) < fabs(GG_OUT(i, j + 1))) GG_OUT(i, j + 1) = cand;
-        }
-        for (int j = ixmax - 1; j > bo.x0; j--) {  // x backward
-            R cand;
-            if (j > ixmin && i < iymax)
-                cand = GG_OUT(i, j) + ((R)sgn(GG_IN(i, j - 1)) * h);
-            else
-                cand = GG_OUT(i, j) + (R)sgn(GG_OUT(i, j - 1)) * h;
-            if (fabs(cand) < fabs(GG_OUT(i, j - 1))) GG_OUT(i, j - 1) = cand;
-        }
-    }
-#undef GG_IN
-#undef GG_OUT
-    __syncthreads();
-    for (int64_t p = threadIdx.x; p < ao; p += blockDim.x) {  // clampValues(-delta, delta)
-        const R v = out[p];
-        if (v < -delta)
-            out[p] = -delta;
-        else if (v > delta)
-            out[p] = delta;
-    }
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256) k_redistance(NetConst C, NetState* S) {
-    const int g = blockIdx.x + 1;
-    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
-    const R* in = phiA_of<R>(S) + S->off_cur[g];
-    R* out = phiB_of<R>(S) + S->off_new[g];
-    redistance_grain<R>(in, S->box_cur[g], out, S->box_new[g], (R)C.h, (R)C.delta);
-}
-
 // LSbox::resizeGrid (src/box.cpp:1408-1485) of one grain (not removed) per
 // block: its distance function on the coarser grid, by bilinear
 // interpolation of the old field (box_cur / off_cur of phiA) at the new grid's

@@ -4,6 +4,7 @@
 #include "gg_corrector.cuh"
 #include "gg_kernels.cuh"
 #include "gg_launch.cuh"
+#include "gg_redist.cuh"
 #include "gg_tangent.cuh"
 #include "gg_warp.cuh"
 
@@ -77,10 +78,33 @@ cudaError_t find_neighbors_launch(const NetConst& C, NetState* dS, const Neighbo
     return cudaGetLastError();
 }
 
+// Dynamic shared memory above the default limit (per device, before the first launch).
+cudaError_t plain_prepare() {
+    const auto allow = [](auto* kernel, size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    cudaError_t e = allow(k_redistance<double, false>, redist_smem<double, false>());
+    if (e == cudaSuccess) e = allow(k_redistance<double, true>, redist_smem<double, true>());
+    if (e == cudaSuccess) e = allow(k_redistance_ts<false>, sizeof(RedistTangentCta<false>));
+    if (e == cudaSuccess) e = allow(k_redistance_ts<true>, sizeof(RedistTangentCta<true>));
+    return e;
+}
+
+void launch_redistance_plain(const NetConst& C, NetState* dS, cudaStream_t s) {
+    k_redistance<double, true><<<C.N, redist_threads<double, true>(), redist_smem<double, true>(), s>>>(C, dS);
+    k_redistance<double, false><<<C.N, kRedistThreads, redist_smem<double, false>(), s>>>(C, dS);
+}
+
+void launch_redistance_tangent(const NetConst& C, NetState* dS, cudaStream_t s) {
+    k_redistance_t<<<C.N, 64, 0, s>>>(C, dS);  // boxes that do not stage
+    k_redistance_ts<true><<<C.N, kRedistTThreads, sizeof(RedistTangentCta<true>), s>>>(C, dS);
+    k_redistance_ts<false><<<C.N, kRedistThreads, sizeof(RedistTangentCta<false>), s>>>(C, dS);
+}
+
 cudaError_t plain_init(const NetConst& C, NetState* dS, const int32_t* d_ids, cudaStream_t s) {
     if (C.N <= 0) return cudaSuccess;
     k_init_phi<double><<<C.N, 256, 0, s>>>(C, dS, d_ids);
-    k_redistance<double><<<C.N, 256, 0, s>>>(C, dS);
+    launch_redistance_plain(C, dS, s);
     k_swap_phi<<<1, 1, 0, s>>>(dS);
     const int gt = 64;
     k_init_contour<double><<<(C.N + gt - 1) / gt, gt, 0, s>>>(C, dS);
@@ -112,7 +136,7 @@ cudaError_t plain_stage_kernel(const NetConst& C, NetState* dS, int which, cudaS
         case 4: k_levelset_w<double><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS); break;
         case 5: k_alloc<<<1, 1024, 0, s>>>(C, dS, 2); break;
         case 6: k_neighbours_w<double><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo)); break;
-        case 7: k_redistance_s<double><<<C.N, kRedistThreads, kRedistSmemBytes, s>>>(C, dS); break;
+        case 7: launch_redistance_plain(C, dS, s); break;
         default: k_finalize<<<1, 1024, 0, s>>>(C, dS, 1); break;
     }
     return cudaGetLastError();
@@ -156,9 +180,9 @@ cudaError_t plain_stages(const NetConst& C, NetState* dS, int stages, cudaStream
         k_alloc<<<1, 1024, 0, s>>>(C, dS, 2);
         k_neighbours_w<double><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo));
         if (tan)
-            k_redistance_t<<<C.N, 64, 0, s>>>(C, dS);
+            launch_redistance_tangent(C, dS, s);
         else
-            k_redistance_s<double><<<C.N, kRedistThreads, kRedistSmemBytes, s>>>(C, dS);
+            launch_redistance_plain(C, dS, s);
         k_finalize<<<1, 1024, 0, s>>>(C, dS, 1);
     }
     return cudaGetLastError();

@@ -26,6 +26,7 @@
 
 #include "gg_corrector.cuh"
 #include "gg_kernels.cuh"
+#include "gg_redist.cuh"
 
 namespace gg {
 namespace {
@@ -508,14 +509,72 @@ __global__ void k_area_t(NetConst C, NetState* S) {
     }
 }
 
-// Redistancing with tangents (replaces k_redistance_s in tangent mode; the
-// value arithmetic is the same, in global memory).  Every output value is a
-// zero-crossing value -dz sgn(slope) = a h s / (c - a) plus steps of +-h, so
-// it carries that crossing's tangent h s (c da - a dc) / (c - a)^2; the -1
-// start values and clamped outputs carry none.
+// Redistancing with tangents.  Every output value is a zero-crossing value
+// -dz sgn(slope) = a h s / (c - a) plus steps of +-h, so it carries that
+// crossing's tangent h s (c da - a dc) / (c - a)^2; the -1 start values and
+// clamped outputs carry none.  The staged sweeps therefore carry only the
+// crossing each value came from, and every output pixel evaluates that
+// crossing's four tangents once at the end (one thread per pixel, instead of
+// four fields carried through the serial sweeps).  kLarge: boxes above
+// kRedistEdge, up to kRedistTEdge.
+constexpr int kRedistTEdge = 120;
+constexpr int kRedistTThreads = 160;
+template <bool kLarge>
+using RedistTangentCta =
+    RedistSmem<double, kLarge ? kRedistTEdge : kRedistEdge, kLarge ? kRedistTThreads : kRedistThreads, true>;
+static_assert(sizeof(RedistTangentCta<false>) <= 75 * 1024);  // 3 CTAs per SM
+static_assert(sizeof(RedistTangentCta<true>) <= 226 * 1024);
+
+__device__ void redistance_tangent(const NetConst& C, NetState* S, int g);
+
+template <bool kLarge>
+__global__ void __launch_bounds__(kLarge ? kRedistTThreads : kRedistThreads) k_redistance_ts(NetConst C, NetState* S) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const int g = blockIdx.x + 1;
+    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
+    const RedistGrain<double> G = redist_grain<double>(C, S, g);
+    const int wo = box_w(G.bo), ho = box_h(G.bo), wi = box_w(G.bi), edge = max(wo, ho);
+    if ((edge > kRedistEdge) != kLarge || edge > kRedistTEdge) return;
+    using M = RedistTangentCta<kLarge>;
+    M& m = *reinterpret_cast<M*>(s_raw);
+    if (!redistance_staged<double, M, true>(G, C.nn, m)) {
+        redistance_tangent(C, S, g);
+        return;
+    }
+    const double* din = reinterpret_cast<const double*>(S->dphiA) + S->off_cur[g];
+    double* dout = reinterpret_cast<double*>(S->dphiB) + S->off_new[g];
+    const int64_t cap = S->phi_cap;
+    for (int p = threadIdx.x; p < wo * ho; p += blockDim.x) {
+        const int r = p / wo, q = M::at(r, p - r * wo);
+        const double x = m.cell[q];
+        const bool clamped = x < -G.delta || x > G.delta;
+        const int from = m.src[q];
+        G.out[p] = clamp_delta(x, G.delta);
+        double d[kNP] = {0, 0, 0, 0};
+        if (!clamped && from >= 0) {
+            const int ci = (from >> 1) / M::kStride - kPad, cj = (from >> 1) % M::kStride - kPad;
+            const int64_t ia = (int64_t)(G.bo.y0 + ci - G.bi.y0) * wi + (G.bo.x0 + cj - G.bi.x0);
+            const int64_t ic = ia + (from & 1 ? 1 : wi);
+            const double a = G.in[ia], c = G.in[ic];
+            const double den = (c - a) * (c - a), s = (double)sgn((c - a) / G.h);
+            if (den > 0)
+                for (int t = 0; t < kNP; ++t)
+                    d[t] = G.h * s * (c * din[t * cap + ia] - a * din[t * cap + ic]) / den;
+        }
+        for (int t = 0; t < kNP; ++t) dout[t * cap + p] = d[t];
+    }
+}
+
+// The same on boxes that do not stage, in device memory, the tangents carried
+// with the values.
 __global__ void __launch_bounds__(64) k_redistance_t(NetConst C, NetState* S) {
     const int g = blockIdx.x + 1;
     if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
+    const Box bo = S->box_new[g];
+    if (max(box_w(bo), box_h(bo)) > kRedistTEdge) redistance_tangent(C, S, g);
+}
+
+__device__ __noinline__ void redistance_tangent(const NetConst& C, NetState* S, int g) {
     const Box bi = S->box_cur[g], bo = S->box_new[g];
     const double h = C.h, delta = C.delta;
     const double* in = phiA_of<double>(S) + S->off_cur[g];

@@ -1174,483 +1174,5 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_second_order_w(NetCons
     }
 }
 
-// LSbox::executeRedistancing (src/box.cpp:1259-1399): one CTA of 64 threads
-// per grain.  The output box is built in shared memory when it fits (16 KB,
-// small enough for many grains per SM), so the four sweeps (threads over
-// columns for y, over rows for x; each column / row a sequential recurrence
-// with the running value carried in a register) never re-read global stores;
-// the input box is read through L1; the result is clamped to +-delta and
-// written back coalesced.
-constexpr int kRedistThreads = 64;
-constexpr int kRedistSmemBytes = 24 * 1024;
-
-// The four directional sweeps of LSbox::executeRedistancing
-// (src/box.cpp:1259-1399) over the new box bo.  The input is read through
-// IN(i, j) = in[(i - in_y0) * si + (j - in_x0)] and is only touched inside
-// the intersection of bi and bo; the output through OUT(i, j) =
-// out[(i - bo.y0) * so + (j - bo.x0)].  One thread per column (y sweeps) or
-// row (x sweeps), carrying the running value in a register.
-template <typename R>
-__device__ void redistance_sweeps_indexed(const R* __restrict__ in, int in_x0, int in_y0, int si, const Box bi,
-                                  R* __restrict__ out, int so, const Box bo, R h) {
-    const int ixmin = (bi.x0 < bo.x0) ? bo.x0 : bi.x0;
-    const int iymin = (bi.y0 < bo.y0) ? bo.y0 : bi.y0;
-    const int ixmax = (bi.x1 < bo.x1) ? bi.x1 : bo.x1;
-    const int iymax = (bi.y1 < bo.y1) ? bi.y1 : bo.y1;
-#define GG_IN(i, j) in[(int64_t)((i) - in_y0) * si + ((j) - in_x0)]
-#define GG_OUT(i, j) out[(int64_t)((i) - bo.y0) * so + ((j) - bo.x0)]
-    // Each recurrence carries its running value in a register; the loads of
-    // the next step (which no store of the current step touches) are issued
-    // one step ahead so their latency overlaps the current step.
-    for (int j = ixmin + (int)threadIdx.x; j < bo.x1; j += blockDim.x) {
-        const bool col_in = j < ixmax;
-        if (iymin < bo.y1 - 1) {  // y forward
-            R cur = GG_OUT(iymin, j);
-            R nxt = GG_OUT(iymin + 1, j);
-            R a = (R)0, c = (R)0;
-            if (col_in && iymin < iymax - 1) {
-                a = GG_IN(iymin, j);
-                c = GG_IN(iymin + 1, j);
-            }
-            for (int i = iymin; i < bo.y1 - 1; i++) {
-                const R nxt_n = i + 2 < bo.y1 ? GG_OUT(i + 2, j) : (R)0;
-                const R c_n = (col_in && i + 1 < iymax - 1) ? GG_IN(i + 2, j) : (R)0;
-                R cand;
-                if (col_in && i < iymax - 1) {
-                    if (a * c <= (R)0.0) {
-                        const R slope = (c - a) / h;
-                        const R dz = -a / slope;
-                        if (fabs(cur) > fabs(dz)) {
-                            cur = -dz * (R)sgn(slope);
-                            GG_OUT(i, j) = cur;
-                        }
-                    }
-                    cand = cur + ((R)sgn(c) * h);
-                } else {
-                    cand = cur + ((R)sgn(nxt) * h);
-                }
-                if (fabs(cand) < fabs(nxt)) {
-                    nxt = cand;
-                    GG_OUT(i + 1, j) = nxt;
-                }
-                cur = nxt;
-                nxt = nxt_n;
-                a = c;
-                c = c_n;
-            }
-        }
-        if (iymax - 1 > bo.y0) {  // y backward
-            R cur = GG_OUT(iymax - 1, j);
-            R prv = GG_OUT(iymax - 2, j);
-            R ip = (col_in && iymax - 1 > iymin) ? GG_IN(iymax - 2, j) : (R)0;
-            for (int i = iymax - 1; i > bo.y0; i--) {
-                const R prv_n = i - 2 >= bo.y0 ? GG_OUT(i - 2, j) : (R)0;
-                const R ip_n = (col_in && i - 1 > iymin) ? GG_IN(i - 2, j) : (R)0;
-                R cand;
-                if (col_in && i > iymin)
-                    cand = cur + ((R)sgn(ip) * h);
-                else
-                    cand = cur + ((R)sgn(prv) * h);
-                if (fabs(cand) < fabs(prv)) {
-                    prv = cand;
-                    GG_OUT(i - 1, j) = prv;
-                }
-                cur = prv;
-                prv = prv_n;
-                ip = ip_n;
-            }
-        }
-    }
-    __syncthreads();
-    for (int i = iymin + (int)threadIdx.x; i < bo.y1; i += blockDim.x) {
-        const bool row_in = i < iymax;
-        if (ixmin < bo.x1 - 1) {  // x forward
-            R cur = GG_OUT(i, ixmin);
-            R nxt = GG_OUT(i, ixmin + 1);
-            R a = (R)0, c = (R)0;
-            if (row_in && ixmin < ixmax - 1) {
-                a = GG_IN(i, ixmin);
-                c = GG_IN(i, ixmin + 1);
-            }
-            for (int j = ixmin; j < bo.x1 - 1; j++) {
-                const R nxt_n = j + 2 < bo.x1 ? GG_OUT(i, j + 2) : (R)0;
-                const R c_n = (row_in && j + 1 < ixmax - 1) ? GG_IN(i, j + 2) : (R)0;
-                R cand;
-                if (j < ixmax - 1 && row_in) {
-                    if (a * c <= (R)0.0) {
-                        const R slope = (c - a) / h;
-                        const R dz = -a / slope;
-                        if (fabs(cur) > fabs(dz)) {
-                            cur = -dz * (R)sgn(slope);
-                            GG_OUT(i, j) = cur;
-                        }
-                    }
-                    cand = cur + ((R)sgn(c) * h);
-                } else {
-                    cand = cur + ((R)sgn(nxt) * h);
-                }
-                if (fabs(cand) < fabs(nxt)) {
-                    nxt = cand;
-                    GG_OUT(i, j + 1) = nxt;
-                }
-                cur = nxt;
-                nxt = nxt_n;
-                a = c;
-                c = c_n;
-            }
-        }
-        if (ixmax - 1 > bo.x0) {  // x backward
-            R cur = GG_OUT(i, ixmax - 1);
-            R prv = GG_OUT(i, ixmax - 2);
-            R ip = (ixmax - 1 > ixmin && row_in) ? GG_IN(i, ixmax - 2) : (R)0;
-            for (int j = ixmax - 1; j > bo.x0; j--) {
-                const R prv_n = j - 2 >= bo.x0 ? GG_OUT(i, j - 2) : (R)0;
-                const R ip_n = (j - 1 > ixmin && row_in) ? GG_IN(i, j - 2) : (R)0;
-                R cand;
-                if (j > ixmin && row_in)
-                    cand = cur + ((R)sgn(ip) * h);
-                else
-                    cand = cur + (R)sgn(prv) * h;
-                if (fabs(cand) < fabs(prv)) {
-                    prv = cand;
-                    GG_OUT(i, j - 1) = prv;
-                }
-                cur = prv;
-                prv = prv_n;
-                ip = ip_n;
-            }
-        }
-    }
-#undef GG_IN
-#undef GG_OUT
-    __syncthreads();
-}
-
-// The four directional sweeps of LSbox::executeRedistancing
-// (src/box.cpp:1259-1399) over the new box bo.  The input is read through
-// IN(i, j) = in[(i - in_y0) * si + (j - in_x0)] and is only touched inside
-// the intersection of bi and bo; the output through OUT(i, j) =
-// out[(i - bo.y0) * so + (j - bo.x0)].  One thread per column (y sweeps) or
-// row (x sweeps), carrying the running value in a register.
-template <typename R>
-__device__ void redistance_sweeps_walk(const R* __restrict__ in, int in_x0, int in_y0, int si, const Box bi,
-                                  R* __restrict__ out, int so, const Box bo, R h) {
-    const int ixmin = (bi.x0 < bo.x0) ? bo.x0 : bi.x0;
-    const int iymin = (bi.y0 < bo.y0) ? bo.y0 : bi.y0;
-    const int ixmax = (bi.x1 < bo.x1) ? bi.x1 : bo.x1;
-    const int iymax = (bi.y1 < bo.y1) ? bi.y1 : bo.y1;
-    // Each recurrence carries its running value in a register and walks the
-    // output (and, inside the intersection, the input) with a pointer; the
-    // loads of the next step (which no store of the current step touches) are
-    // issued one step ahead so their latency overlaps the current step.  Each
-    // sweep is split where the input's region ends, so the loop bodies carry
-    // no per-step region test.
-    // y sweeps: one thread per column, stride so / si between steps
-    for (int j = ixmin + (int)threadIdx.x; j < bo.x1; j += blockDim.x) {
-        const bool col_in = j < ixmax;
-        R* const ocol = out + (j - bo.x0);
-        const R* const icol = in + (j - in_x0);
-        if (iymin < bo.y1 - 1) {  // y forward
-            const int a_end = col_in ? min(iymax - 1, bo.y1 - 1) : iymin;  // steps that see the input
-            R* po = ocol + (iymin - bo.y0) * so;
-            const R* pi = icol + (iymin - in_y0) * si;
-            R cur = po[0];
-            R nxt = po[so];
-            int i = iymin;
-            if (i < a_end) {
-                R a = pi[0], c = pi[si];
-                for (; i < a_end; i++) {
-                    const R nxt_n = i + 2 < bo.y1 ? po[2 * so] : (R)0;
-                    const R c_n = i + 1 < iymax - 1 ? pi[2 * si] : (R)0;
-                    if (a * c <= (R)0.0) {
-                        const R slope = (c - a) / h;
-                        const R dz = -a / slope;
-                        if (fabs(cur) > fabs(dz)) {
-                            cur = -dz * (R)sgn(slope);
-                            po[0] = cur;
-                        }
-                    }
-                    const R cand = cur + ((R)sgn(c) * h);
-                    if (fabs(cand) < fabs(nxt)) {
-                        nxt = cand;
-                        po[so] = nxt;
-                    }
-                    cur = nxt;
-                    nxt = nxt_n;
-                    a = c;
-                    c = c_n;
-                    po += so;
-                    pi += si;
-                }
-            }
-            for (; i < bo.y1 - 1; i++) {
-                const R nxt_n = i + 2 < bo.y1 ? po[2 * so] : (R)0;
-                const R cand = cur + ((R)sgn(nxt) * h);
-                if (fabs(cand) < fabs(nxt)) {
-                    nxt = cand;
-                    po[so] = nxt;
-                }
-                cur = nxt;
-                nxt = nxt_n;
-                po += so;
-            }
-        }
-        if (iymax - 1 > bo.y0) {  // y backward
-            const int a_end = col_in ? iymin : iymax - 1;  // steps i > a_end see the input
-            R* po = ocol + (iymax - 1 - bo.y0) * so;
-            R cur = po[0];
-            R prv = po[-so];
-            int i = iymax - 1;
-            if (i > a_end) {
-                const R* pi = icol + (iymax - 2 - in_y0) * si;  // IN(i - 1)
-                R ip = pi[0];
-                for (; i > a_end; i--) {
-                    const R prv_n = i - 2 >= bo.y0 ? po[-2 * so] : (R)0;
-                    const R ip_n = i - 1 > iymin ? pi[-si] : (R)0;
-                    const R cand = cur + ((R)sgn(ip) * h);
-                    if (fabs(cand) < fabs(prv)) {
-                        prv = cand;
-                        po[-so] = prv;
-                    }
-                    cur = prv;
-                    prv = prv_n;
-                    ip = ip_n;
-                    po -= so;
-                    pi -= si;
-                }
-            }
-            for (; i > bo.y0; i--) {
-                const R prv_n = i - 2 >= bo.y0 ? po[-2 * so] : (R)0;
-                const R cand = cur + ((R)sgn(prv) * h);
-                if (fabs(cand) < fabs(prv)) {
-                    prv = cand;
-                    po[-so] = prv;
-                }
-                cur = prv;
-                prv = prv_n;
-                po -= so;
-            }
-        }
-    }
-    __syncthreads();
-    // x sweeps: one thread per row, unit stride between steps
-    for (int i = iymin + (int)threadIdx.x; i < bo.y1; i += blockDim.x) {
-        const bool row_in = i < iymax;
-        R* const orow = out + (int64_t)(i - bo.y0) * so;
-        const R* const irow = in + (int64_t)(i - in_y0) * si;
-        if (ixmin < bo.x1 - 1) {  // x forward
-            const int a_end = row_in ? min(ixmax - 1, bo.x1 - 1) : ixmin;
-            R* po = orow + (ixmin - bo.x0);
-            const R* pi = irow + (ixmin - in_x0);
-            R cur = po[0];
-            R nxt = po[1];
-            int j = ixmin;
-            if (j < a_end) {
-                R a = pi[0], c = pi[1];
-                for (; j < a_end; j++) {
-                    const R nxt_n = j + 2 < bo.x1 ? po[2] : (R)0;
-                    const R c_n = j + 1 < ixmax - 1 ? pi[2] : (R)0;
-                    if (a * c <= (R)0.0) {
-                        const R slope = (c - a) / h;
-                        const R dz = -a / slope;
-                        if (fabs(cur) > fabs(dz)) {
-                            cur = -dz * (R)sgn(slope);
-                            po[0] = cur;
-                        }
-                    }
-                    const R cand = cur + ((R)sgn(c) * h);
-                    if (fabs(cand) < fabs(nxt)) {
-                        nxt = cand;
-                        po[1] = nxt;
-                    }
-                    cur = nxt;
-                    nxt = nxt_n;
-                    a = c;
-                    c = c_n;
-                    ++po;
-                    ++pi;
-                }
-            }
-            for (; j < bo.x1 - 1; j++) {
-                const R nxt_n = j + 2 < bo.x1 ? po[2] : (R)0;
-                const R cand = cur + ((R)sgn(nxt) * h);
-                if (fabs(cand) < fabs(nxt)) {
-                    nxt = cand;
-                    po[1] = nxt;
-                }
-                cur = nxt;
-                nxt = nxt_n;
-                ++po;
-            }
-        }
-        if (ixmax - 1 > bo.x0) {  // x backward
-            const int a_end = row_in ? ixmin : ixmax - 1;
-            R* po = orow + (ixmax - 1 - bo.x0);
-            R cur = po[0];
-            R prv = po[-1];
-            int j = ixmax - 1;
-            if (j > a_end) {
-                const R* pi = irow + (ixmax - 2 - in_x0);  // IN(i, j - 1)
-                R ip = pi[0];
-                for (; j > a_end; j--) {
-                    const R prv_n = j - 2 >= bo.x0 ? po[-2] : (R)0;
-                    const R ip_n = j - 1 > ixmin ? pi[-1] : (R)0;
-                    const R cand = cur + ((R)sgn(ip) * h);
-                    if (fabs(cand) < fabs(prv)) {
-                        prv = cand;
-                        po[-1] = prv;
-                    }
-                    cur = prv;
-                    prv = prv_n;
-                    ip = ip_n;
-                    --po;
-                    --pi;
-                }
-            }
-            for (; j > bo.x0; j--) {
-                const R prv_n = j - 2 >= bo.x0 ? po[-2] : (R)0;
-                const R cand = cur + (R)sgn(prv) * h;
-                if (fabs(cand) < fabs(prv)) {
-                    prv = cand;
-                    po[-1] = prv;
-                }
-                cur = prv;
-                prv = prv_n;
-                --po;
-            }
-        }
-    }
-    __syncthreads();
-}
-
-// The FP32 (batched) form walks pointers with each sweep split where the
-// input's region ends (fewer instructions: 0.75 -> 0.68 ms on the 20,000-grain
-// workload); the FP64 (plain) form keeps indexed accesses with per-step region
-// tests, which the compiler schedules better for doubles (1.75 ms against
-// 2.33 ms).  Both evaluate the same expressions in the same order.
-template <typename R>
-__device__ __forceinline__ void redistance_sweeps(const R* __restrict__ in, int in_x0, int in_y0, int si, const Box bi,
-                                                  R* __restrict__ out, int so, const Box bo, R h) {
-    if constexpr (sizeof(R) == 4)
-        redistance_sweeps_walk<R>(in, in_x0, in_y0, si, bi, out, so, bo, h);
-    else
-        redistance_sweeps_indexed<R>(in, in_x0, in_y0, si, bi, out, so, bo, h);
-}
-
-// LSbox::executeRedistancing of grain g by the whole CTA (any block size).
-// When both fit in kSmem bytes, the input over the intersection of the old
-// and new boxes and the output box are staged in shared memory with odd row
-// strides (so the row-wise sweeps hit distinct banks); a larger box keeps
-// only its output there, and the largest stay in global memory.
-// clearValues(-1) before, clampValues(-delta, delta) after.
-template <typename R, int kSmem>
-__device__ void redistance_grain_s(const NetConst& C, NetState* S, int g, unsigned char* s_raw) {
-    const R* in_g = phiA_of<R>(S) + S->off_cur[g];
-    R* out_g = phiB_of<R>(S) + S->off_new[g];
-    const Box bi = S->box_cur[g], bo = S->box_new[g];
-    const R h = (R)C.h, delta = (R)C.delta;
-    const int wi = box_w(bi), wo = box_w(bo), ho = box_h(bo);
-    const int64_t ao = box_area(bo);
-    const int ixmin = (bi.x0 < bo.x0) ? bo.x0 : bi.x0;
-    const int iymin = (bi.y0 < bo.y0) ? bo.y0 : bi.y0;
-    const int ixmax = (bi.x1 < bo.x1) ? bi.x1 : bo.x1;
-    const int iymax = (bi.y1 < bo.y1) ? bi.y1 : bo.y1;
-    const int wI = ixmax > ixmin ? ixmax - ixmin : 0, hI = iymax > iymin ? iymax - iymin : 0;
-    const int so = wo | 1, sI = wI | 1;
-    const bool fits = (int64_t)sizeof(R) * ((int64_t)so * ho + (int64_t)sI * hI) <= kSmem;
-    if (fits) {
-        R* out = reinterpret_cast<R*>(s_raw);
-        R* in = out + so * ho;
-        // row by row, eight loads in flight per thread
-        const R* src = in_g + (int64_t)(iymin - bi.y0) * wi + (ixmin - bi.x0);
-        for (int r0 = 0; r0 < hI; r0 += 8)
-            for (int c = threadIdx.x; c < wI; c += blockDim.x) {
-                R v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = r0 + u < hI ? src[(int64_t)(r0 + u) * wi + c] : (R)0;
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (r0 + u < hI) in[(r0 + u) * sI + c] = v[u];
-            }
-        for (int p = threadIdx.x; p < so * ho; p += blockDim.x) out[p] = (R)-1.0;  // clearValues(-1)
-        __syncthreads();
-        redistance_sweeps<R>(in, ixmin, iymin, sI, bi, out, so, bo, h);
-        for (int r = 0; r < ho; ++r)  // clampValues(-delta, delta)
-            for (int c = threadIdx.x; c < wo; c += blockDim.x) {
-                R v = out[r * so + c];
-                if (v < -delta)
-                    v = -delta;
-                else if (v > delta)
-                    v = delta;
-                out_g[(int64_t)r * wo + c] = v;
-            }
-    } else if ((int64_t)sizeof(R) * so * ho <= kSmem) {  // output staged, input read in place
-        R* out = reinterpret_cast<R*>(s_raw);
-        for (int p = threadIdx.x; p < so * ho; p += blockDim.x) out[p] = (R)-1.0;
-        __syncthreads();
-        redistance_sweeps<R>(in_g, bi.x0, bi.y0, wi, bi, out, so, bo, h);
-        for (int r = 0; r < ho; ++r)
-            for (int c = threadIdx.x; c < wo; c += blockDim.x) {
-                R v = out[r * so + c];
-                if (v < -delta)
-                    v = -delta;
-                else if (v > delta)
-                    v = delta;
-                out_g[(int64_t)r * wo + c] = v;
-            }
-    } else {
-        for (int64_t p = threadIdx.x; p < ao; p += blockDim.x) out_g[p] = (R)-1.0;
-        __syncthreads();
-        redistance_sweeps<R>(in_g, bi.x0, bi.y0, wi, bi, out_g, wo, bo, h);
-        for (int64_t p = threadIdx.x; p < ao; p += blockDim.x) {
-            R v = out_g[p];
-            if (v < -delta)
-                v = -delta;
-            else if (v > delta)
-                v = delta;
-            out_g[p] = v;
-        }
-    }
-}
-
-// Large boxes (batched form, size bin above NetConst::big_edge, 128 unless
-// tuned): k_redistance_big takes them with 256 threads and up to 200 KB of
-// shared memory, so a 168^2 box is staged whole and a 256^2 one sweeps 4x as
-// many columns at a time.  At 128 the bin starts above the largest boxes of a
-// uniform-seed Voronoi network (edge <= 98 at 25 cells per grain), so there
-// it is an empty launch.
-constexpr int kRedistBigThreads = 256;
-constexpr int kRedistBigSmemBytes = 200 * 1024;
-
-// One CTA of 64 threads per grain: every grain in the plain form; in the
-// batched form those whose box edge is at most C.big_edge.
-template <typename R>
-__global__ void __launch_bounds__(kRedistThreads) k_redistance_s(NetConst C, NetState* S) {
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    const int g = grain_at(S, blockIdx.x);
-    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
-    if (S->order && box_w(S->box_cur[g]) > C.big_edge) return;  // the large-box bin
-    redistance_grain_s<R, kRedistSmemBytes>(C, S, g, s_raw);
-}
-
-// The large-box bin of the batched form: a persistent grid walks the work
-// queue (largest boxes first) and stops at the first existing grain at or
-// below C.big_edge; k_redistance_s follows it on the same stream (run
-// side by side, the two measured slower: the 64-thread kernel's blocks take
-// the SMs first).
-__global__ void __launch_bounds__(kRedistBigThreads) k_redistance_big(NetConst C, NetState* S) {
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    if (!S->order) return;
-    for (int slot = blockIdx.x; slot < C.N; slot += gridDim.x) {
-        const int g = S->order[slot];
-        // a grain that vanished in this step's level set keeps its place in
-        // the queue; existing grains are in descending box edge
-        if (C.state[g] != G_EXISTS || halted(S)) continue;
-        if (box_w(S->box_cur[g]) <= C.big_edge) return;
-        redistance_grain_s<float, kRedistBigSmemBytes>(C, S, g, s_raw);
-        __syncthreads();  // the next grain reuses the shared buffers
-    }
-}
-
 }  // namespace
 }  // namespace gg
