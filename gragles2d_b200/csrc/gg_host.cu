@@ -116,7 +116,7 @@ struct gg_ctx {
     bool stats_fresh = false;
     uint32_t* h_status = nullptr;
     cudaEvent_t ev_done = nullptr;
-    LaunchCfg cfg{256, 256, 128, 64};
+    LaunchCfg cfg{256, 64, {nullptr, nullptr}, nullptr};
 
     cudaGraphExec_t graph = nullptr;
     bool sectors_stale = false;    // batched form: the corrector's sectors need a rebuild before the next step
@@ -833,6 +833,9 @@ int gg_create(const gg_params* p, int device, gg_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking);
     for (int k = 0; k < kStepForks && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&c->fork[k], cudaEventDisableTiming);
+    c->cfg.side[0] = c->stream2;
+    c->cfg.side[1] = c->stream3;
+    c->cfg.ev = c->fork;
     if (e != cudaSuccess) {
         c->err = std::string("stream/event: ") + cudaGetErrorString(e);
         *out = c;

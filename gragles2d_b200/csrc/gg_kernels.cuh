@@ -22,106 +22,6 @@ __device__ __forceinline__ R* phiB_of(NetState* S) {
 }
 
 // ---------------------------------------------------------------------------
-// Convolution, plain form (src/box.cpp:622-695 with the FFTW transforms
-// evaluated as separable direct DFTs in a fixed summation order): one CTA
-// per grain, phi_t (arena A) -> convolved field (arena B, same box).
-// Row r2c, column DFT and Gaussian multiply, inverse column DFT, row c2r.
-// ---------------------------------------------------------------------------
-template <typename R>
-__global__ void __launch_bounds__(256) k_conv_dft(NetConst C, NetState* S, int tk = -1) {
-    const int g = blockIdx.x + 1;
-    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
-    const Box bx = S->box_cur[g];
-    const int n = box_w(bx);
-    if (n <= 0) return;
-    if (n != box_h(bx) || n > C.tmax) {
-        if (threadIdx.x == 0) set_status(S, n > C.tmax ? S_TABLE_RANGE : S_INDEX);
-        return;
-    }
-    const int half = n / 2 + 1;
-    // tk >= 0: the same (linear) convolution of tangent field tk
-    const R* in = (tk < 0 ? phiA_of<R>(S) : reinterpret_cast<R*>(S->dphiA) + tk * S->phi_cap) + S->off_cur[g];
-    R* out = (tk < 0 ? phiB_of<R>(S) : reinterpret_cast<R*>(S->dphiB) + tk * S->phi_cap) + S->off_cur[g];
-    R* s1 = reinterpret_cast<R*>(S->spec) + S->soff_cur[g];  // n x half complex
-    R* s2 = s1 + 2 * (int64_t)n * half;                        // n x half complex
-    const double* w = C.tw + 2 * C.tw_off[n];
-    const double* G = C.gk + C.gk_off[n];
-    const int tot = n * half;
-
-    // rows: T[r][f] = sum_c x[r][c] w^(f c)
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int r = idx / half, f = idx - r * half;
-        R re = 0, im = 0;
-        const R* xr = in + r * n;
-        int k = 0;
-        for (int c = 0; c < n; ++c) {
-            const R v = xr[c];
-            re = re + v * (R)w[2 * k];
-            im = im + v * (R)w[2 * k + 1];
-            k += f;
-            if (k >= n) k -= n;
-        }
-        s1[2 * idx] = re;
-        s1[2 * idx + 1] = im;
-    }
-    __syncthreads();
-    // columns: Y[q][f] = sum_r T[r][f] w^(q r), then * G(f, min(q, n-q))
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int q = idx / half, f = idx - q * half;
-        R re = 0, im = 0;
-        int k = 0;
-        for (int r = 0; r < n; ++r) {
-            const R a = s1[2 * (r * half + f)], b = s1[2 * (r * half + f) + 1];
-            const R wc = (R)w[2 * k], ws = (R)w[2 * k + 1];
-            re = re + (a * wc - b * ws);
-            im = im + (a * ws + b * wc);
-            k += q;
-            if (k >= n) k -= n;
-        }
-        const int j2 = q < n - q ? q : n - q;
-        const R gv = (R)G[f * half + j2];
-        s2[2 * idx] = re * gv;
-        s2[2 * idx + 1] = im * gv;
-    }
-    __syncthreads();
-    // inverse columns: T[r][f] = sum_q Y[q][f] conj(w)^(q r)
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int r = idx / half, f = idx - r * half;
-        R re = 0, im = 0;
-        int k = 0;
-        for (int q = 0; q < n; ++q) {
-            const R a = s2[2 * (q * half + f)], b = s2[2 * (q * half + f) + 1];
-            const R wc = (R)w[2 * k], ws = -(R)w[2 * k + 1];
-            re = re + (a * wc - b * ws);
-            im = im + (a * ws + b * wc);
-            k += r;
-            if (k >= n) k -= n;
-        }
-        s1[2 * idx] = re;
-        s1[2 * idx + 1] = im;
-    }
-    __syncthreads();
-    // rows c2r: x[r][c] = T0 + 2 sum_f Re(T_f e^{+i..}) (+ Nyquist)
-    const int hmax = (n - 1) / 2;
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-        const int r = idx / n, c = idx - r * n;
-        const R* t = s1 + 2 * (int64_t)r * half;
-        R acc = t[0];
-        int k = 0;
-        for (int f = 1; f <= hmax; ++f) {
-            k += c;
-            if (k >= n) k -= n;
-            acc = acc + (R)2.0 * (t[2 * f] * (R)w[2 * k] + t[2 * f + 1] * (R)w[2 * k + 1]);
-        }
-        if ((n & 1) == 0) {
-            const R nyq = t[2 * (n / 2)];
-            acc = acc + ((c & 1) ? -nyq : nyq);
-        }
-        out[idx] = acc;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // LSbox::computeSecondOrderNeighbours (src/box.cpp:1027-1068): one thread per
 // grain.  New list = existing members of the previous list, in order, then
 // members of their lists whose (convolution) boxes intersect ours, first

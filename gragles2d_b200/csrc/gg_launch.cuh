@@ -21,10 +21,11 @@ enum : int {
 };
 
 struct LaunchCfg {
-    int conv_threads;
     int compare_threads;
-    int redist_threads;
     int grain_threads;  // one-thread-per-grain kernels
+    // further streams and events of the context, for launches that run side by side
+    cudaStream_t side[2];
+    cudaEvent_t* ev;
 };
 
 // Declared per form; defined in gg_plain.cu / gg_batched.cu.

@@ -2,6 +2,7 @@
 // so every sum, product and quotient rounds exactly as the reference's
 // host arithmetic does.
 #include "gg_corrector.cuh"
+#include "gg_dft.cuh"
 #include "gg_kernels.cuh"
 #include "gg_launch.cuh"
 #include "gg_redist.cuh"
@@ -83,11 +84,34 @@ cudaError_t plain_prepare() {
     const auto allow = [](auto* kernel, size_t bytes) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
-    cudaError_t e = allow(k_redistance<double, false>, redist_smem<double, false>());
+    cudaError_t e = allow(k_conv_dft_s<0>, dft_smem(DftBin<0>::kHigh));
+    if (e == cudaSuccess) e = allow(k_conv_dft_s<1>, dft_smem(DftBin<1>::kHigh));
+    if (e == cudaSuccess) e = allow(k_conv_dft_s<2>, dft_smem(DftBin<2>::kHigh));
+    if (e == cudaSuccess) e = allow(k_redistance<double, false>, redist_smem<double, false>());
     if (e == cudaSuccess) e = allow(k_redistance<double, true>, redist_smem<double, true>());
     if (e == cudaSuccess) e = allow(k_redistance_ts<false>, sizeof(RedistTangentCta<false>));
     if (e == cudaSuccess) e = allow(k_redistance_ts<true>, sizeof(RedistTangentCta<true>));
     return e;
+}
+
+// The distance field's convolution, and with `tangents` that of its four
+// tangent fields.
+cudaError_t launch_convolution_plain(const NetConst& C, NetState* dS, cudaStream_t s, const LaunchCfg& cfg,
+                                     bool tangents) {
+    const dim3 grid(C.N, tangents ? 1 + kNP : 1);
+    cudaError_t e;
+    if ((e = cudaEventRecord(cfg.ev[0], s)) != cudaSuccess) return e;
+    for (int k = 0; k < 2; ++k)
+        if ((e = cudaStreamWaitEvent(cfg.side[k], cfg.ev[0], 0)) != cudaSuccess) return e;
+    k_conv_dft_s<2><<<grid, DftBin<2>::kThreads, dft_smem(DftBin<2>::kHigh), cfg.side[0]>>>(C, dS);
+    for (int tk = -1; tk < (tangents ? kNP : 0); ++tk) k_conv_dft<<<C.N, 256, 0, cfg.side[0]>>>(C, dS, tk);
+    k_conv_dft_s<1><<<grid, DftBin<1>::kThreads, dft_smem(DftBin<1>::kHigh), cfg.side[1]>>>(C, dS);
+    k_conv_dft_s<0><<<grid, DftBin<0>::kThreads, dft_smem(DftBin<0>::kHigh), s>>>(C, dS);
+    for (int k = 0; k < 2; ++k) {
+        if ((e = cudaEventRecord(cfg.ev[1 + k], cfg.side[k])) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(s, cfg.ev[1 + k], 0)) != cudaSuccess) return e;
+    }
+    return cudaGetLastError();
 }
 
 void launch_redistance_plain(const NetConst& C, NetState* dS, cudaStream_t s) {
@@ -129,7 +153,7 @@ cudaError_t plain_stage_kernel(const NetConst& C, NetState* dS, int which, cudaS
     const int wblocks = (C.N + kGrainsPerBlock - 1) / kGrainsPerBlock;
     (void)gblocks;
     switch (which) {
-        case 0: k_conv_dft<double><<<C.N, cfg.conv_threads, 0, s>>>(C, dS); break;
+        case 0: return launch_convolution_plain(C, dS, s, cfg, false);
         case 1: if (!C.isotropic) k_corrector<double><<<C.N, 128, 0, s>>>(C, dS); break;
         case 2: k_second_order_w<<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS); break;
         case 3: k_compare<double><<<C.N, cfg.compare_threads, 0, s>>>(C, dS); break;
@@ -158,9 +182,8 @@ cudaError_t plain_stages(const NetConst& C, NetState* dS, int stages, cudaStream
     // so it runs first
     const bool tan = C.dvol != nullptr;
     if (stages & ST_CONV) {
-        k_conv_dft<double><<<C.N, cfg.conv_threads, 0, s>>>(C, dS);
-        if (tan)
-            for (int tk = 0; tk < kNP; ++tk) k_conv_dft<double><<<C.N, cfg.conv_threads, 0, s>>>(C, dS, tk);
+        cudaError_t ec = launch_convolution_plain(C, dS, s, cfg, tan);
+        if (ec != cudaSuccess) return ec;
         if (!C.isotropic) {
             if (tan) k_corrector_t<<<C.N, 128, 0, s>>>(C, dS);
             cudaError_t e = plain_corrector(C, dS, s);
