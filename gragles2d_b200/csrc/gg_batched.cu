@@ -295,13 +295,6 @@ __device__ void build_buckets(VertexBuckets<kPts>& B, const float2* P32, int npt
     __syncthreads();
 }
 
-__device__ __forceinline__ double dist2_rn(double px, double py, const CPoint& q) {
-    const double ex = px - q.x, ey = py - q.y;
-    return __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey));
-}
-
-__device__ __forceinline__ float tie_margin(float d, float eps_c) { return (sqrtf(d) + 1.f) * eps_c + d * 1e-6f; }
-
 constexpr unsigned kKeyIndexBits = 10;
 constexpr unsigned kKeyIndexMask = (1u << kKeyIndexBits) - 1u;
 static_assert(kCorrStagedPts <= kCorrBigPts && kCorrBigPts <= (1 << kKeyIndexBits), "vertex index must fit the key");
@@ -438,62 +431,6 @@ __device__ __forceinline__ int segment_step(const float2* P32, const CPoint* P, 
     const float lam = before ? lb : la;
     *out_lambda = fminf(fmaxf(lam, 0.f), 1.f);
     return before ? nv - 1 : nearest;
-}
-
-// Sectors of every grain for the next corrector (batched form), built one
-// step ahead so that the corrector's warps do not wait on the serial build:
-// the same build as the plain corrector's (prepare_sectors: segment lengths,
-// neighbour table, junction weights, then setPointsOnBoundary and the
-// constant / interpolating sectors, src/grainBoundary.cpp:233-342,
-// src/contourSector.cpp), one 32-thread CTA per grain.  kCur: from the roles
-// the step just produced (contour, junctions, IDLocal of this step, run after
-// the neighbour characteristics are computed), which become the previous
-// ones at the end of the step; else from the previous roles (after
-// initialisation, grid coarsening or new neighbour lists).
-template <bool kCur>
-__global__ void __launch_bounds__(32) k_sectors(NetConst C, NetState* S) {
-    const int g = grain_at(S, blockIdx.x);
-    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
-    __shared__ SectorSet sec;
-    __shared__ double jw[64];
-    __shared__ uint32_t s_st;
-    __shared__ double s_per;
-    __shared__ NbTable nbt;
-    __shared__ int jl[64], jr[64];
-    const int64_t coff = kCur ? S->coff_cur[g] : S->coff_prev[g];
-    const CPoint* P = (kCur ? S->contCur : S->contPrev) + coff;
-    const int size = kCur ? S->cn_cur[g] : S->cn_prev[g];
-    SectorPack* pk = reinterpret_cast<SectorPack*>(C.secpack) + g;
-    if (size < 2) {
-        if (threadIdx.x == 0) {
-            pk->nconst = 0;
-            pk->ninterp = 0;
-        }
-        return;
-    }
-    // segment lengths: the corrector's scratch at this contour's offsets (no
-    // corrector reads it while this kernel runs; a global buffer leaves room
-    // for more CTAs per SM than a shared one)
-    double* seg = S->segPrev + coff;
-    const Box ib = kCur ? S->box_cur[g] : S->box_prev[g];
-    const uint32_t* idl = kCur ? S->idCur + S->off_cur[g] : S->idPrev + S->off_prev[g];
-    const Junction* J = (kCur ? S->jCur : S->jPrev) + (int64_t)g * C.jmax;
-    const int nj = min(kCur ? S->jn_cur[g] : S->jn_prev[g], 64);
-    prepare_sectors_view(C, S, g, P, size, seg, sec, jw, &s_st, &s_per, nbt, jl, jr, ib, idl, J, nj);
-    const int nc = sec.nconst, ni = sec.ninterp;
-    if (threadIdx.x == 0) {
-        pk->nconst = nc;
-        pk->ninterp = ni;
-    }
-    for (int c = threadIdx.x; c < nc; c += blockDim.x) pk->cw[c] = sec.cs[c].weight;
-    for (int c = threadIdx.x; c < ni; c += blockDim.x) pk->is[c] = sec.is[c];
-    for (int q = threadIdx.x; q < size - 1; q += blockDim.x) {
-        int sid;
-        double acc;
-        seg_table_entry(sec, seg, size, q, &sid, &acc);
-        C.segsec[coff + q] = (int16_t)sid;
-        C.segacc[coff + q] = (float)acc;
-    }
 }
 
 // Shared memory of one CTA of the batched corrector.
@@ -822,7 +759,7 @@ size_t batched_sector_pack_bytes() { return sizeof(SectorPack); }
 
 cudaError_t batched_sectors(const NetConst& C, NetState* dS, cudaStream_t s) {
     if (C.N <= 0) return cudaSuccess;
-    k_sectors<false><<<C.N, 32, 0, s>>>(C, dS);
+    k_sectors<false, float><<<C.N, 32, 0, s>>>(C, dS);
     return cudaGetLastError();
 }
 
@@ -852,7 +789,7 @@ cudaError_t batched_stage_kernel(const NetConst& C, NetState* dS, int which, cud
         case 5: k_alloc<<<1, 1024, 0, s>>>(C, dS, 1); break;
         case 6:
             k_neighbours_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo));
-            k_sectors<true><<<C.N, 32, 0, s>>>(C, dS);
+            k_sectors<true, float><<<C.N, 32, 0, s>>>(C, dS);
             break;
         case 7: launch_redistance(C, dS, s); break;
         default:
@@ -879,7 +816,7 @@ cudaError_t batched_stages(const NetConst& C, NetState* dS, int stages, cudaStre
     if (stages & ST_REDIST) {
         k_alloc<<<1, 1024, 0, s>>>(C, dS, 1);
         k_neighbours_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo));
-        k_sectors<true><<<C.N, 32, 0, s>>>(C, dS);
+        k_sectors<true, float><<<C.N, 32, 0, s>>>(C, dS);
         launch_redistance(C, dS, s);
         k_finalize<<<1, 1024, 0, s>>>(C, dS, 1);
         k_order<<<1, 1024, 0, s>>>(C, dS);
@@ -917,7 +854,7 @@ cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, 
     if ((e = cudaEventRecord(ev[5], s3)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s2, ev[2], 0)) != cudaSuccess) return e;
     k_neighbours_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s2>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo));
-    k_sectors<true><<<C.N, 32, 0, s2>>>(C, dS);  // the next step's sectors
+    k_sectors<true, float><<<C.N, 32, 0, s2>>>(C, dS);  // the next step's sectors
     if ((e = cudaEventRecord(ev[3], s2)) != cudaSuccess) return e;
     launch_redistance_main(C, dS, s);
     if ((e = cudaStreamWaitEvent(s, ev[3], 0)) != cudaSuccess) return e;

@@ -40,17 +40,6 @@ struct SectorSet {
     InterpSector is[kMaxInterpSectors];
 };
 
-// Per contour segment: the sector getWeight would pick (first constant
-// sector containing it, else first interpolating sector, else none) and, for
-// an interpolating sector, the partial sum of segment lengths from the
-// sector's right point up to the segment, accumulated in the same order as
-// ContourSector::getWeight (src/contourSector.cpp:242-246).
-constexpr int kSegTable = 512;
-struct SegTable {
-    short sector[kSegTable];  // >= 0 constant, <= -2 interpolating (-2 - q), -1 none
-    double acc[kSegTable];
-};
-
 // characteristics lookup of ExplicitGrainBoundary::getDirectNeighbourCaracteristic
 // (src/grainBoundary.cpp:561-571): by grain ID; a removed grain matches
 // nothing; absent -> default (energy 1, mobility 1).
@@ -561,7 +550,11 @@ __device__ void build_sectors_warp(const NetConst& C, const NbTable& T, const CP
     __syncwarp();
 }
 
-// Segment q's entry of the per-segment table (see SegTable).
+// Segment q's entry of the per-segment table: the sector getWeight would pick
+// (>= 0: the first constant sector containing it, else <= -2: -2 - the first
+// interpolating one, else -1) and, for an interpolating sector, the partial sum
+// of segment lengths from the sector's right point up to the segment, in the
+// order of ContourSector::getWeight (src/contourSector.cpp:242-246).
 __device__ __forceinline__ void seg_table_entry(const SectorSet& S, const double* seg, int size, int q, int* sid_out,
                                                 double* acc_out) {
     const int real = size - 1;
@@ -590,18 +583,7 @@ __device__ __forceinline__ void seg_table_entry(const SectorSet& S, const double
     *acc_out = acc;
 }
 
-__device__ void build_seg_table(const SectorSet& S, const double* seg, int size, SegTable& T) {
-    for (int q = threadIdx.x; q < size - 1; q += blockDim.x) {
-        int sid;
-        double acc;
-        seg_table_entry(S, seg, size, q, &sid, &acc);
-        T.sector[q] = (short)sid;
-        T.acc[q] = acc;
-    }
-}
-
-// The sectors of a grain as the batched corrector reads them, built one step
-// ahead (k_sectors): the constant sectors' weights and the interpolating
+// The sectors of a grain as the correctors read them (from k_sectors): the constant sectors' weights and the interpolating
 // sectors; the per-segment table lives beside the contour (NetConst::segsec,
 // segacc at the contour's offsets).
 struct SectorPack {
@@ -611,38 +593,20 @@ struct SectorPack {
     InterpSector is[kMaxInterpSectors];
 };
 
-// ExplicitGrainBoundary::getWeight (src/grainBoundary.cpp:344-363) for one pixel.
-__device__ __forceinline__ double pixel_weight(const NetConst& C, const NbTable& T, const CPoint* P,
-                                               const double* seg, int size, const SectorSet& S,
-                                               const SegTable* ST, const uint32_t* idl, const Box& ib, int i, int j,
-                                               uint32_t* status) {
-    double lambda = 0.0;
-    const int segment = project_to_boundary(P, size, (double)j, (double)i, &lambda);
-    const int real = size - 1;
-    int sid = -1;
-    double interpolator = 0;
-    if (ST) {
-        sid = ST->sector[segment];
-        if (sid <= -2) interpolator = ST->acc[segment];
-    } else {
-        for (int q = 0; q < S.nconst && sid == -1; q++)
-            if (within(S.cs[q].left, S.cs[q].right, real, segment)) sid = q;
-        for (int q = 0; q < S.ninterp && sid == -1; q++)
-            if (within(S.is[q].left, S.is[q].right, real, segment)) sid = -2 - q;
-        if (sid <= -2) {
-            int it = 0;
-            for (int k = S.is[-2 - sid].right; k != segment; k = wrap_next(k, real)) {
-                interpolator += seg[k];
-                if (++it > size) break;
-            }
-        }
-    }
-    if (sid >= 0) return S.cs[sid].weight;
+// ExplicitGrainBoundary::getWeight (src/grainBoundary.cpp:344-363) for one pixel
+// projected onto `segment` at lambda; sid and acc are the segment's sector and
+// arc length (see seg_table_entry), cw and is the sectors.
+__device__ __forceinline__ double segment_weight(const NetConst& C, const NbTable& T, const CPoint* P, int real, int sid,
+                                                 double acc, const double* cw, const InterpSector* is, int segment,
+                                                 double lambda, const uint32_t* idl, const Box& ib, int i, int j,
+                                                 uint32_t* status) {
+    if (sid >= 0) return cw[sid];
     if (sid == -1) return table_weight_at(T, idl, ib, i, j, status);
-    const InterpSector& s = S.is[-2 - sid];
+    const InterpSector& s = is[-2 - sid];
     const int k = segment;
     const int kn = wrap_next(k, real);
     const double ax = (P[kn].x - P[k].x) * lambda, ay = (P[kn].y - P[k].y) * lambda;
+    double interpolator = acc;
     interpolator += sqrt(ax * ax + ay * ay);
     interpolator /= s.length;
     if (interpolator < 0) interpolator = 0;
@@ -705,54 +669,181 @@ __device__ void prepare_sectors_view(const NetConst& C, NetState* S, int g, cons
     __syncthreads();
 }
 
-template <typename R>
-__global__ void __launch_bounds__(128) k_corrector(NetConst C, NetState* S) {
-    const int g = blockIdx.x + 1;
-    if (g > C.N || C.state[g] != G_EXISTS || C.regular[g] == 0 || S->loop == 0 || halted(S)) return;
+// Sectors of every grain for the corrector, in a kernel of their own so that
+// the corrector's warps do not wait on the serial build: one step ahead in the
+// batched form, beside the convolution in the plain form.  The build is
+// prepare_sectors' (segment lengths,
+// neighbour table, junction weights, then setPointsOnBoundary and the
+// constant / interpolating sectors, src/grainBoundary.cpp:233-342,
+// src/contourSector.cpp), one 32-thread CTA per grain.  kCur: from the roles
+// the step just produced (contour, junctions, IDLocal of this step, run after
+// the neighbour characteristics are computed), which become the previous
+// ones at the end of the step; else from the previous roles (after
+// initialisation, grid coarsening or new neighbour lists).
+// A: the type of the per-segment arc lengths (segacc of the form).
+template <bool kCur, typename A>
+__global__ void __launch_bounds__(32) k_sectors(NetConst C, NetState* S) {
+    const int g = grain_at(S, blockIdx.x);
+    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
     __shared__ SectorSet sec;
     __shared__ double jw[64];
     __shared__ uint32_t s_st;
     __shared__ double s_per;
     __shared__ NbTable nbt;
-    __shared__ double s_seg[kSegShared];
-    __shared__ SegTable stab;
     __shared__ int jl[64], jr[64];
-    const CPoint* P = S->contPrev + S->coff_prev[g];
-    const int size = S->cn_prev[g];
-    if (size < 2) return;
-    double* seg = size - 1 <= kSegShared ? s_seg : S->segPrev + S->coff_prev[g];
-    const Box ib = S->box_prev[g];
-    const uint32_t* idl = S->idPrev + S->off_prev[g];
-    prepare_sectors(C, S, g, P, size, seg, sec, jw, &s_st, &s_per, nbt, jl, jr);
-    const bool tabled = size - 1 <= kSegTable;
-    if (tabled) build_seg_table(sec, seg, size, stab);
-    __syncthreads();
-    const Box bo = S->box_cur[g];
-    const int x0 = ib.x0 < bo.x0 ? bo.x0 : ib.x0;
-    const int y0 = ib.y0 < bo.y0 ? bo.y0 : ib.y0;
-    const int x1 = ib.x1 > bo.x1 ? bo.x1 : ib.x1;
-    const int y1 = ib.y1 > bo.y1 ? bo.y1 : ib.y1;
-    if (x1 <= x0 || y1 <= y0) return;
-    const int w = x1 - x0;
-    const int64_t cnt = (int64_t)w * (y1 - y0);
-    const R* in = phiA_of<R>(S) + S->off_cur[g];
-    R* out = phiB_of<R>(S) + S->off_cur[g];
-    const int wo = box_w(bo);
-    const R delta = (R)C.delta;
-    uint32_t st = 0;
-    for (int64_t p = threadIdx.x; p < cnt; p += blockDim.x) {
-        const int i = y0 + (int)(p / w), j = x0 + (int)(p % w);
-        const int64_t k = (int64_t)(i - bo.y0) * wo + (j - bo.x0);
-        const R val = in[k];
-        if (val > -delta) {
-            const double weight = pixel_weight(C, nbt, P, seg, size, sec, tabled ? &stab : nullptr, idl, ib, i, j, &st);
-            out[k] = (R)((double)val + ((double)out[k] - (double)val) * weight * 1.0);
-        } else {
-            out[k] = -delta;
+    const int64_t coff = kCur ? S->coff_cur[g] : S->coff_prev[g];
+    const CPoint* P = (kCur ? S->contCur : S->contPrev) + coff;
+    const int size = kCur ? S->cn_cur[g] : S->cn_prev[g];
+    SectorPack* pk = reinterpret_cast<SectorPack*>(C.secpack) + g;
+    if (size < 2) {
+        if (threadIdx.x == 0) {
+            pk->nconst = 0;
+            pk->ninterp = 0;
         }
-        if (C.stored || C.magnetic) out[k] = subtract_driving_forces<R>(C, nbt, idl, ib, i, j, out[k], &st);
+        return;
     }
-    if (st) set_status(S, st);
+    // segment lengths: the corrector's scratch at this contour's offsets (no
+    // corrector reads it while this kernel runs; a global buffer leaves room
+    // for more CTAs per SM than a shared one)
+    double* seg = S->segPrev + coff;
+    const Box ib = kCur ? S->box_cur[g] : S->box_prev[g];
+    const uint32_t* idl = kCur ? S->idCur + S->off_cur[g] : S->idPrev + S->off_prev[g];
+    const Junction* J = (kCur ? S->jCur : S->jPrev) + (int64_t)g * C.jmax;
+    const int nj = min(kCur ? S->jn_cur[g] : S->jn_prev[g], 64);
+    prepare_sectors_view(C, S, g, P, size, seg, sec, jw, &s_st, &s_per, nbt, jl, jr, ib, idl, J, nj);
+    const int nc = sec.nconst, ni = sec.ninterp;
+    if (threadIdx.x == 0) {
+        pk->nconst = nc;
+        pk->ninterp = ni;
+    }
+    for (int c = threadIdx.x; c < nc; c += blockDim.x) pk->cw[c] = sec.cs[c].weight;
+    for (int c = threadIdx.x; c < ni; c += blockDim.x) pk->is[c] = sec.is[c];
+    for (int q = threadIdx.x; q < size - 1; q += blockDim.x) {
+        int sid;
+        double acc;
+        seg_table_entry(sec, seg, size, q, &sid, &acc);
+        C.segsec[coff + q] = (int16_t)sid;
+        if constexpr (sizeof(A) == 4) C.segacc[coff + q] = (float)acc;
+        else C.segacc64[coff + q] = acc;
+    }
+}
+
+__device__ __forceinline__ double dist2_rn(double px, double py, const CPoint& q) {
+    const double ex = px - q.x, ey = py - q.y;
+    return __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey));
+}
+
+__device__ __forceinline__ float tie_margin(float d, float eps_c) { return (sqrtf(d) + 1.f) * eps_c + d * 1e-6f; }
+
+// Nearest contour vertex of projectToGrainBondary (src/grainBoundary.cpp:
+// 365-381) for the pixels of one 8 x 4 tile per warp, as FP64 takes it.  From
+// the tile's centre the lanes measure every vertex once, in FP32 on the
+// staged contour; only a vertex within the smallest of these distances plus
+// the tile's diameter can be the nearest of one of its pixels, and those (25 of
+// 130 in a typical tile beside the boundary) go to the warp's list in index
+// order.  Each lane then measures the listed ones: keys of distance bits with
+// the list position in the low bits, the two smallest kept.  Where they lie
+// within twice the FP32 rounding (tie_margin), the lane measures the listed
+// vertices within the margin again in FP64, lowest index first (the
+// reference's strict < over ascending k).
+constexpr int kTileList = 128;
+constexpr unsigned kTileMask = kTileList - 1u;
+
+// sp: the contour less (ox, oy) in FP32; span: the largest coordinate of sp
+// and of the pixels in magnitude.  All lanes call it; returns the vertex of a
+// `need` lane's pixel (px, py), or -1 if none lies within the reference's
+// initial distance (1e6).
+__device__ __forceinline__ int nearest_vertex_tile(const float2* sp, const CPoint* P, int npts, int tx, int ty, int px,
+                                                   int py, int ox, int oy, float span, bool need, float4* list) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const float cx = (float)(tx - ox) + 3.5f, cy = (float)(ty - oy) + 1.5f;
+    float best = 3e38f;
+    for (int k = lane; k < npts; k += 32) {
+        const float dx = cx - sp[k].x, dy = cy - sp[k].y;
+        best = fminf(best, fmaf(dy, dy, dx * dx));
+    }
+    best = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(best)));
+    // the tile's diameter is 2 x 3.8079; the slack covers FP32's rounding
+    const float reach = sqrtf(best) + 7.6158f + 1e-3f + 4e-6f * span;
+    const float reach2 = reach * reach;
+    int n = 0;
+    for (int k0 = 0; k0 < npts; k0 += 32) {
+        const int k = k0 + lane;
+        float2 v = make_float2(0.f, 0.f);
+        bool in = false;
+        if (k < npts) {
+            v = sp[k];
+            const float dx = cx - v.x, dy = cy - v.y;
+            in = fmaf(dy, dy, dx * dx) <= reach2;
+        }
+        const unsigned m = __ballot_sync(FULL, in);
+        const int pos = n + __popc(m & ((1u << lane) - 1u));
+        if (in && pos < kTileList) list[pos] = make_float4(v.x, v.y, __int_as_float(k), 0.f);
+        n += __popc(m);
+    }
+    __syncwarp();
+    const float fx = (float)(px - ox), fy = (float)(py - oy);
+    int nearest = -1;
+    if (n <= kTileList) {
+        unsigned k1 = 0xffffffffu, k2 = 0xffffffffu;
+#pragma unroll 4
+        for (int q = 0; q < n; ++q) {
+            const float4 v = list[q];
+            const float dx = fx - v.x, dy = fy - v.y;
+            const unsigned key = (__float_as_uint(fmaf(dy, dy, dx * dx)) & ~kTileMask) | (unsigned)q;
+            k2 = min(k2, max(k1, key));
+            k1 = min(k1, key);
+        }
+        // k1 | mask is at least the distance of k1's vertex
+        const float d1 = __uint_as_float(k1 | kTileMask);
+        const float thr = d1 + tie_margin(d1, 8.f * 5.9604645e-8f * (span + 2.f));
+        if (need && (k2 != 0xffffffffu && __uint_as_float(k2 & ~kTileMask) <= thr || d1 > 0.99e6f)) {
+            const double dpx = (double)px, dpy = (double)py;
+            double closest = 1000000.0;
+            for (int q = 0; q < n; ++q) {
+                const float dx = fx - list[q].x, dy = fy - list[q].y;
+                if (fmaf(dy, dy, dx * dx) > thr) continue;
+                const int k = __float_as_int(list[q].z);
+                const double d = dist2_rn(dpx, dpy, P[k]);
+                if (d < closest) {
+                    closest = d;
+                    nearest = k;
+                }
+            }
+        } else {
+            nearest = __float_as_int(list[k1 & kTileMask].z);
+        }
+    } else if (need) {
+        const double dpx = (double)px, dpy = (double)py;
+        double closest = 1000000.0;
+        for (int k = 0; k < npts; ++k) {
+            const double d = dist2_rn(dpx, dpy, P[k]);
+            if (d < closest) {
+                closest = d;
+                nearest = k;
+            }
+        }
+    }
+    __syncwarp();  // the list is the next tile's
+    return nearest;
+}
+
+// Contour points staged in FP32 by the plain form's correctors.
+constexpr int kCorrPts = 512;
+
+// Largest |coordinate| of the staged contour and of a box of the given size,
+// by the whole CTA (ends with a barrier).
+__device__ __forceinline__ float staged_span(const float2* sp, int size, int w, int h) {
+    __shared__ unsigned s_span;
+    if (threadIdx.x == 0) s_span = __float_as_uint((float)max(w, h));
+    __syncthreads();
+    float v = 0.f;
+    for (int k = threadIdx.x; k < size; k += blockDim.x) v = fmaxf(v, fmaxf(fabsf(sp[k].x), fabsf(sp[k].y)));
+    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_span, top);
+    __syncthreads();
+    return __uint_as_float(s_span);
 }
 
 }  // namespace

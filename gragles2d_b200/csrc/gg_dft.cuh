@@ -240,10 +240,12 @@ __global__ void __launch_bounds__(DftBin<kBin>::kThreads, DftBin<kBin>::kPerSm) 
                     reinterpret_cast<const double2*>(C.tw) + C.tw_off[n], C.gk + C.gk_off[n], s_raw);
 }
 
-// Boxes above kDftEdge, one output per thread, the spectra in the
-// grain's scratch in device memory (so one field after the other); also
-// reports a box that has no tables.
-__global__ void __launch_bounds__(256) k_conv_dft(NetConst C, NetState* S, int tk) {
+// Boxes above kDftEdge, one output per thread, the spectra in the grain's
+// scratch in device memory (so the distance field and the `tangents` tangent
+// fields one after the other); also reports a box that has no tables.
+__device__ void conv_dft_box(const NetConst& C, const double* in, double* out, double* s1, int n);
+
+__global__ void __launch_bounds__(256) k_conv_dft(NetConst C, NetState* S, int tangents) {
     const int g = blockIdx.x + 1;
     if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
     const Box bx = S->box_cur[g];
@@ -254,12 +256,18 @@ __global__ void __launch_bounds__(256) k_conv_dft(NetConst C, NetState* S, int t
         return;
     }
     if (n <= kDftEdge) return;
+    double* s1 = reinterpret_cast<double*>(S->spec) + S->soff_cur[g];  // 2 x n x half complex
+    conv_dft_box(C, phiA_of<double>(S) + S->off_cur[g], phiB_of<double>(S) + S->off_cur[g], s1, n);
+    for (int tk = 0; tk < tangents; ++tk) {
+        __syncthreads();
+        conv_dft_box(C, reinterpret_cast<double*>(S->dphiA) + tk * S->phi_cap + S->off_cur[g],
+                     reinterpret_cast<double*>(S->dphiB) + tk * S->phi_cap + S->off_cur[g], s1, n);
+    }
+}
+
+__device__ void conv_dft_box(const NetConst& C, const double* in, double* out, double* s1, int n) {
     const int half = n / 2 + 1;
-    // tk >= 0: the same (linear) convolution of tangent field tk
-    const double* in = (tk < 0 ? phiA_of<double>(S) : reinterpret_cast<double*>(S->dphiA) + tk * S->phi_cap) + S->off_cur[g];
-    double* out = (tk < 0 ? phiB_of<double>(S) : reinterpret_cast<double*>(S->dphiB) + tk * S->phi_cap) + S->off_cur[g];
-    double* s1 = reinterpret_cast<double*>(S->spec) + S->soff_cur[g];  // n x half complex
-    double* s2 = s1 + 2 * (int64_t)n * half;                           // n x half complex
+    double* s2 = s1 + 2 * (int64_t)n * half;
     const double* w = C.tw + 2 * C.tw_off[n];
     const double* G = C.gk + C.gk_off[n];
     const int tot = n * half;

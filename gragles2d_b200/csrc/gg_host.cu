@@ -1422,14 +1422,16 @@ int gg_distance_initialisation(gg_ctx* c) {
         S.phiA = pa;
         S.phiB = pb;
         S.spec = sp_;
-        // sectors built one step ahead for the corrector
+        ALLOC(C.segacc, cont_cap);
+        c->sectors_stale = true;  // built one step ahead
+    }
+    if (!plain || !C.isotropic) {  // the corrector's sectors
         char* pk;
         ALLOC(pk, batched_sector_pack_bytes() * (size_t)(N + 1));
         C.secpack = pk;
         ALLOC(C.segsec, cont_cap);
-        ALLOC(C.segacc, cont_cap);
-        c->sectors_stale = true;
     }
+    if (plain && !C.isotropic) ALLOC_UNZEROED(C.segacc64, cont_cap);
     (void)rsz;
     ALLOC(S.idPrev, phi_cap);
     ALLOC(S.idCur, phi_cap);

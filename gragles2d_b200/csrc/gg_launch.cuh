@@ -34,7 +34,6 @@ cudaError_t plain_prepare();
 cudaError_t plain_init(const NetConst& C, NetState* dS, const int32_t* d_ids, cudaStream_t s);
 // distance initialisation from the loaded polygons (contour input)
 cudaError_t plain_init_polygon(const NetConst& C, NetState* dS, cudaStream_t s);
-cudaError_t plain_corrector(const NetConst& C, NetState* dS, cudaStream_t s);
 cudaError_t batched_stages(const NetConst& C, NetState* dS, int stages, cudaStream_t s, const LaunchCfg& cfg);
 // The whole batched step for graph capture on s, with the independent stages
 // (second-order lists beside convolution + corrector, volume / energy /
