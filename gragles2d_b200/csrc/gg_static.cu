@@ -26,12 +26,20 @@ namespace {
 
 constexpr int kMaxN = GG_STATIC_CONV_MAX_N;
 constexpr int kMaxHalf = kMaxN / 2 + 1;
-// Layout of the scratch (doubles): two spectra of n x (n/2+1) complex values,
-// the twiddles exp(-2 pi i k / n) for k < n, the multipliers G(i2, j2).
-constexpr size_t kSpecDoubles = 2 * 2 * (size_t)kMaxN * kMaxHalf;
-constexpr size_t kTwDoubles = 2 * (size_t)kMaxN;
-constexpr size_t kGDoubles = (size_t)kMaxHalf * kMaxHalf;
-constexpr size_t kScratchDoubles = kSpecDoubles + kTwDoubles + kGDoubles;
+// Layout of the scratch (doubles): two spectra of n x (n/2+1) complex values.
+constexpr size_t kSpecDoubles = 2 * (size_t)kMaxN * kMaxHalf;
+constexpr size_t kScratchDoubles = 2 * kSpecDoubles;
+
+// The tables of one call travel as kernel parameters (19 KB at most, of the
+// 32 KB a kernel takes): no copy to the device, and nothing of the caller's
+// frame to wait for.
+struct Twiddles {
+    double2 w[kMaxN];  // exp(-2 pi i k / n)
+};
+struct Multipliers {
+    double g[kMaxHalf * (kMaxHalf + 1) / 2];  // G(i, j) = G(j, i) at j (j + 1) / 2 + i, i <= j
+};
+static_assert(sizeof(Twiddles) + sizeof(Multipliers) < 32000);
 
 // The fixed device scratch.  In host code this name is only a host-side
 // stand-in for the symbol, not a device address: the address used by kernels
@@ -83,83 +91,103 @@ int scratch_on_device(double** out) {
     return GG_OK;
 }
 
-// One CTA: rows r2c, columns DFT times G, inverse columns, rows c2r; the same
-// sums in the same order as the plain convolution stage.
-__global__ void __launch_bounds__(256) k_conv_box_static(const double* __restrict__ in, double* __restrict__ out,
-                                                         int n, double* __restrict__ scratch) {
-    const int half = n / 2 + 1;
-    double* s1 = scratch;
-    double* s2 = scratch + 2 * (size_t)n * half;
-    const double* w = scratch + kSpecDoubles;
-    const double* G = w + kTwDoubles;
-    const int tot = n * half;
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int r = idx / half, f = idx - r * half;
-        double re = 0, im = 0;
-        const double* xr = in + (size_t)r * n;
-        int k = 0;
-        for (int c = 0; c < n; ++c) {
-            const double v = xr[c];
-            re = re + v * w[2 * k];
-            im = im + v * w[2 * k + 1];
-            k += f;
-            if (k >= n) k -= n;
-        }
-        s1[2 * idx] = re;
-        s1[2 * idx + 1] = im;
-    }
+// The same sums in the same order as the plain convolution stage, one output
+// per thread, spread over the device: a CTA per row, per column (forward,
+// multiplier and back), per row.  Each sum is a chain of up to 128 additions
+// (8 cycles each), so a transform takes 2 to 3 us whatever its parallelism; one
+// CTA for the whole box took 1.3 ms at n = 128.  A whole call: 1374 -> 54 us at
+// n = 128 (half of it the host's multipliers), 76 -> 30 us at n = 45.
+constexpr int kThreads = kMaxN;
+
+__device__ __forceinline__ void stage_twiddles(const Twiddles& t, double2* w, int n) {
+    for (int k = threadIdx.x; k < n; k += blockDim.x) w[k] = t.w[k];
+}
+
+__global__ void __launch_bounds__(kThreads) k_box_rows(const double* __restrict__ in, int n, double2* __restrict__ T,
+                                                       const __grid_constant__ Twiddles tw) {
+    __shared__ double2 w[kMaxN];
+    __shared__ double x[kMaxN];
+    const int half = n / 2 + 1, r = blockIdx.x, f = threadIdx.x;
+    stage_twiddles(tw, w, n);
+    if (f < n) x[f] = in[(size_t)r * n + f];
     __syncthreads();
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int q = idx / half, f = idx - q * half;
+    if (f >= half) return;
+    double re = 0, im = 0;
+    int k = 0;
+#pragma unroll 4
+    for (int c = 0; c < n; ++c) {
+        const double2 e = w[k];
+        re = re + x[c] * e.x;
+        im = im + x[c] * e.y;
+        k += f;
+        if (k >= n) k -= n;
+    }
+    T[(size_t)r * half + f] = make_double2(re, im);
+}
+
+__global__ void __launch_bounds__(kThreads) k_box_columns(const double2* __restrict__ T, int n,
+                                                          double2* __restrict__ out, const __grid_constant__ Twiddles tw,
+                                                          const __grid_constant__ Multipliers G) {
+    __shared__ double2 w[kMaxN], a[kMaxN], y[kMaxN];
+    const int half = n / 2 + 1, f = blockIdx.x, q = threadIdx.x;
+    stage_twiddles(tw, w, n);
+    if (q < n) a[q] = T[(size_t)q * half + f];
+    __syncthreads();
+    if (q < n) {
         double re = 0, im = 0;
         int k = 0;
+#pragma unroll 4
         for (int r = 0; r < n; ++r) {
-            const double a = s1[2 * (r * half + f)], b = s1[2 * (r * half + f) + 1];
-            const double wc = w[2 * k], ws = w[2 * k + 1];
-            re = re + (a * wc - b * ws);
-            im = im + (a * ws + b * wc);
+            const double2 v = a[r], e = w[k];
+            re = re + (v.x * e.x - v.y * e.y);
+            im = im + (v.x * e.y + v.y * e.x);
             k += q;
             if (k >= n) k -= n;
         }
-        const int j2 = q < n - q ? q : n - q;
-        const double gv = G[f * half + j2];
-        s2[2 * idx] = re * gv;
-        s2[2 * idx + 1] = im * gv;
+        const int j2 = q < n - q ? q : n - q, lo = f < j2 ? f : j2, hi = f < j2 ? j2 : f;
+        const double gv = G.g[hi * (hi + 1) / 2 + lo];
+        y[q] = make_double2(re * gv, im * gv);
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int r = idx / half, f = idx - r * half;
+    if (q < n) {  // thread q is row r now
         double re = 0, im = 0;
         int k = 0;
-        for (int q = 0; q < n; ++q) {
-            const double a = s2[2 * (q * half + f)], b = s2[2 * (q * half + f) + 1];
-            const double wc = w[2 * k], ws = -w[2 * k + 1];
-            re = re + (a * wc - b * ws);
-            im = im + (a * ws + b * wc);
-            k += r;
+#pragma unroll 4
+        for (int p = 0; p < n; ++p) {
+            const double2 v = y[p], e = w[k];
+            const double ws = -e.y;
+            re = re + (v.x * e.x - v.y * ws);
+            im = im + (v.x * ws + v.y * e.x);
+            k += q;
             if (k >= n) k -= n;
         }
-        s1[2 * idx] = re;
-        s1[2 * idx + 1] = im;
+        out[(size_t)q * half + f] = make_double2(re, im);
     }
+}
+
+__global__ void __launch_bounds__(kThreads) k_box_back(const double2* __restrict__ T, int n, double* __restrict__ out,
+                                                       const __grid_constant__ Twiddles tw) {
+    __shared__ double2 w[kMaxN], t[kMaxHalf];
+    const int half = n / 2 + 1, r = blockIdx.x, c = threadIdx.x;
+    stage_twiddles(tw, w, n);
+    if (c < half) t[c] = T[(size_t)r * half + c];
     __syncthreads();
+    if (c >= n) return;
     const int hmax = (n - 1) / 2;
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-        const int r = idx / n, c = idx - r * n;
-        const double* t = s1 + 2 * (size_t)r * half;
-        double acc = t[0];
-        int k = 0;
-        for (int f = 1; f <= hmax; ++f) {
-            k += c;
-            if (k >= n) k -= n;
-            acc = acc + 2.0 * (t[2 * f] * w[2 * k] + t[2 * f + 1] * w[2 * k + 1]);
-        }
-        if ((n & 1) == 0) {
-            const double nyq = t[2 * (n / 2)];
-            acc = acc + ((c & 1) ? -nyq : nyq);
-        }
-        out[idx] = acc;
+    double acc = t[0].x;
+    int k = 0;
+#pragma unroll 4
+    for (int f = 1; f <= hmax; ++f) {
+        k += c;
+        if (k >= n) k -= n;
+        const double2 e = w[k];
+        acc = acc + 2.0 * (t[f].x * e.x + t[f].y * e.y);
     }
+    if ((n & 1) == 0) {
+        const double nyq = t[n / 2].x;
+        acc = acc + ((c & 1) ? -nyq : nyq);
+    }
+    out[(size_t)r * n + c] = acc;
 }
 
 }  // namespace
@@ -169,30 +197,30 @@ extern "C" int gg_convolve_box_static(const double* d_in, double* d_out, int32_t
     if (n < 1 || n > kMaxN) return GG_E_INVALID;
     if (!d_in || !d_out || real_domain_size < 1 || !(dt > 0)) return GG_E_INVALID;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // A call copies its tables from this stack frame and waits for the
-    // stream, neither of which a stream capture admits: a capturing stream
-    // is refused before anything is issued on it, so the capture stays valid.
+    // A call waits for the stream, which a stream capture does not admit: a
+    // capturing stream is refused before anything is issued on it, so the
+    // capture stays valid.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) return cuda_error();
     if (cap != cudaStreamCaptureStatusNone) return GG_E_INVALID;
     double* scratch = nullptr;
     const int rc = scratch_on_device(&scratch);
     if (rc != GG_OK) return rc;
-    // Tables for this n, built on the host stack (no heap allocation) and
-    // copied into the scratch; every value the kernel reads is rewritten by
-    // this call, so nothing has to be cleared between calls.
-    double tables[kTwDoubles + kGDoubles];
+    // Tables for this n, built on the host stack (no heap allocation); every
+    // value the kernels read is written by this call.
     const int half = n / 2 + 1;
-    for (int k = 0; k < n; ++k) twiddle(n, k, &tables[2 * k], &tables[2 * k + 1]);
-    double* G = tables + kTwDoubles;
-    for (int i2 = 0; i2 < half; ++i2)
-        for (int j2 = 0; j2 < half; ++j2) G[i2 * half + j2] = gaussian_multiplier(n, i2, j2, dt, real_domain_size);
-    cudaError_t e = cudaMemcpyAsync(scratch + kSpecDoubles, tables, sizeof(tables), cudaMemcpyHostToDevice, s);
+    Twiddles tw;
+    for (int k = 0; k < n; ++k) twiddle(n, k, &tw.w[k].x, &tw.w[k].y);
+    Multipliers G;
+    for (int j2 = 0; j2 < half; ++j2)  // the argument is i2^2 + j2^2: symmetric
+        for (int i2 = 0; i2 <= j2; ++i2) G.g[j2 * (j2 + 1) / 2 + i2] = gaussian_multiplier(n, i2, j2, dt, real_domain_size);
+    double2* const s1 = reinterpret_cast<double2*>(scratch);
+    double2* const s2 = s1 + kSpecDoubles / 2;
+    k_box_rows<<<n, kThreads, 0, s>>>(d_in, n, s1, tw);
+    k_box_columns<<<half, kThreads, 0, s>>>(s1, n, s2, tw, G);
+    k_box_back<<<n, kThreads, 0, s>>>(s2, n, d_out, tw);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error();
-    k_conv_box_static<<<1, 256, 0, s>>>(d_in, d_out, n, scratch);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_error();
-    // The host table buffer lives on this stack frame: wait for the copy.
     e = cudaStreamSynchronize(s);
     return e == cudaSuccess ? GG_OK : cuda_error();
 }
