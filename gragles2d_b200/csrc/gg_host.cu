@@ -1280,6 +1280,12 @@ int gg_distance_initialisation(gg_ctx* c) {
     C.jmax = 48;
     C.tmax = tmax;
     C.big_edge = 64;
+    // Few boxes: eight warps each, so that they fill the device; many: two, so
+    // that a box's list loads and its last tiles hide behind more other boxes
+    // (us of the stage with 256 / 128 / 64 threads: 60 boxes 21 / 31 / 51, 1,000
+    // 33 / 42 / 70, 2,000 64 / 65 / 113, 20,000 591 / 427 / 401, 100,000 clustered
+    // 3,394 / 2,424 / 2,230; FP64 5,000 201 / 196 / 235).
+    c->cfg.compare_threads = N < 2048 ? 256 : (N < 8192 ? 128 : 64);
     C.conv_smem_edge = 64;
     C.isotropic = P.is_isotropic_network ? 1 : 0;
     C.use_mobility_model = P.use_mobility_model;
@@ -1684,7 +1690,7 @@ int gg_autotune(gg_ctx* c, int32_t loop, int32_t steps_per_candidate, gg_tuning*
         return GG_OK;
     };
     if ((rc = tune(&c->C.big_edge, {48, 56, 64})) != GG_OK) return rc;
-    if ((rc = tune(&c->cfg.compare_threads, {128, 256})) != GG_OK) return rc;  // k_compare: at most 256
+    if ((rc = tune(&c->cfg.compare_threads, {64, 128, 256})) != GG_OK) return rc;  // k_compare: at most 256
     if ((rc = tune(&c->C.conv_smem_edge, {48, 64, 96, 128})) != GG_OK) return rc;
     if (c->graph) {
         cudaGraphExecDestroy(c->graph);
