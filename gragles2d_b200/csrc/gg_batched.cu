@@ -715,21 +715,43 @@ cudaError_t batched_prepare(int tmax) {
     return cudaSuccess;
 }
 
-// The large-box bin of the redistancing, at the device's highest priority
-// (beside the main kernel its CTAs are placed first).
-void launch_redistance_big(const NetConst& C, NetState* dS, cudaStream_t s) {
-    using L = RedistLarge<float>;
+// Launch with the device's highest priority: beside another kernel its CTAs
+// are placed first.
+template <class K>
+void launch_first(K kernel, int grid, int threads, size_t smem, cudaStream_t s, const NetConst& C, NetState* dS) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(C.N < L::kPerSm * g_big_grid ? C.N : L::kPerSm * g_big_grid);
-    cfg.blockDim = dim3(L::kThreads);
-    cfg.dynamicSmemBytes = redist_smem<float, true>();
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributePriority;
     attr[0].val.priority = g_high_priority;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_redistance_big, C, dS);
+    cudaLaunchKernelEx(&cfg, kernel, C, dS);
+}
+
+// The largest boxes' level set (8 one-warp CTAs per SM) and the others'.
+void launch_levelset_big(const NetConst& C, NetState* dS, cudaStream_t s) {
+    launch_first(k_levelset_big<float>, C.N < 8 * g_big_grid ? C.N : 8 * g_big_grid, 32, 0, s, C, dS);
+}
+
+void launch_levelset_main(const NetConst& C, NetState* dS, cudaStream_t s) {
+    k_levelset_w<float><<<(C.N + kGrainsPerBlock - 1) / kGrainsPerBlock, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
+}
+
+// Both on one stream (the graph runs them on two).
+void launch_levelset(const NetConst& C, NetState* dS, cudaStream_t s) {
+    launch_levelset_big(C, dS, s);
+    launch_levelset_main(C, dS, s);
+}
+
+// The large-box bin of the redistancing.
+void launch_redistance_big(const NetConst& C, NetState* dS, cudaStream_t s) {
+    using L = RedistLarge<float>;
+    const int most = L::kPerSm * g_big_grid;
+    launch_first(k_redistance_big, C.N < most ? C.N : most, L::kThreads, redist_smem<float, true>(), s, C, dS);
 }
 
 void launch_redistance_main(const NetConst& C, NetState* dS, cudaStream_t s) {
@@ -751,6 +773,7 @@ cudaError_t batched_init(const NetConst& C, NetState* dS, const int32_t* d_ids, 
     launch_redistance(C, dS, s);
     cudaError_t e = swap_phi(dS, s);
     if (e != cudaSuccess) return e;
+    k_init_contour_big<float><<<C.N, 32, 0, s>>>(C, dS);
     k_init_contour_w<float><<<(C.N + kGrainsPerBlock - 1) / kGrainsPerBlock, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
     return cudaGetLastError();
 }
@@ -785,7 +808,7 @@ cudaError_t batched_stage_kernel(const NetConst& C, NetState* dS, int which, cud
         case 1: if (!C.isotropic) launch_corrector_f(C, dS, s); break;
         case 2: k_second_order_w<<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS); break;
         case 3: k_compare<float><<<C.N, cfg.compare_threads, 0, s>>>(C, dS); break;
-        case 4: k_levelset_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS); break;
+        case 4: launch_levelset(C, dS, s); break;
         case 5: k_alloc<<<1, 1024, 0, s>>>(C, dS, 1); break;
         case 6:
             k_neighbours_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo));
@@ -812,7 +835,7 @@ cudaError_t batched_stages(const NetConst& C, NetState* dS, int stages, cudaStre
     }
     if (stages & ST_SECOND) k_second_order_w<<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
     if (stages & ST_COMPARE) k_compare<float><<<C.N, cfg.compare_threads, 0, s>>>(C, dS);
-    if (stages & ST_LEVELSET) k_levelset_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
+    if (stages & ST_LEVELSET) launch_levelset(C, dS, s);
     if (stages & ST_REDIST) {
         k_alloc<<<1, 1024, 0, s>>>(C, dS, 1);
         k_neighbours_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo));
@@ -844,7 +867,13 @@ cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, 
     if ((e = cudaEventRecord(ev[1], s2)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s, ev[1], 0)) != cudaSuccess) return e;
     k_compare<float><<<C.N, cfg.compare_threads, 0, s>>>(C, dS);
-    k_levelset_w<float><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
+    // the largest boxes' contours beside the others
+    if ((e = cudaEventRecord(ev[0], s)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(s3, ev[0], 0)) != cudaSuccess) return e;
+    launch_levelset_big(C, dS, s3);
+    if ((e = cudaEventRecord(ev[5], s3)) != cudaSuccess) return e;
+    launch_levelset_main(C, dS, s);
+    if ((e = cudaStreamWaitEvent(s, ev[5], 0)) != cudaSuccess) return e;
     k_alloc<<<1, 1024, 0, s>>>(C, dS, 1);
     // volume / energy / neighbours (contours, lists) and the next step's
     // sectors beside redistancing (fields)

@@ -1279,7 +1279,11 @@ int gg_distance_initialisation(gg_ctx* c) {
     C.nbmax = 48;
     C.jmax = 48;
     C.tmax = tmax;
-    C.big_edge = 64;
+    // The small redistancing kernel stages new boxes up to 64 cells.  A box that
+    // grows past that in the step it is taken takes 50 us on its own, so few
+    // boxes leave it more room (stage at 60 / 64: 1,000 grains 46 / 62 us, 2,000
+    // 60 / 97, 20,000 365 / 341).
+    C.big_edge = N < 8192 ? 60 : 64;
     // Few boxes: eight warps each, so that they fill the device; many: two, so
     // that a box's list loads and its last tiles hide behind more other boxes
     // (us of the stage with 256 / 128 / 64 threads: 60 boxes 21 / 31 / 51, 1,000
@@ -1689,7 +1693,7 @@ int gg_autotune(gg_ctx* c, int32_t loop, int32_t steps_per_candidate, gg_tuning*
         *knob = chosen;
         return GG_OK;
     };
-    if ((rc = tune(&c->C.big_edge, {48, 56, 64})) != GG_OK) return rc;
+    if ((rc = tune(&c->C.big_edge, {48, 56, 60, 64})) != GG_OK) return rc;
     if ((rc = tune(&c->cfg.compare_threads, {64, 128, 256})) != GG_OK) return rc;  // k_compare: at most 256
     if ((rc = tune(&c->C.conv_smem_edge, {48, 64, 96, 128})) != GG_OK) return rc;
     if (c->graph) {

@@ -854,29 +854,6 @@ __global__ void __launch_bounds__(256) k_init_phi(NetConst C, NetState* S, const
     }
 }
 
-template <typename R>
-__global__ void k_init_contour(NetConst C, NetState* S) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
-    const Box bx = S->box_cur[g];
-    Field<R> f{phiA_of<R>(S) + S->off_cur[g], bx};
-    const uint32_t* idl = S->idPrev + S->off_prev[g];
-    ContourOut o{S->contPrev + S->coff_prev[g], S->ccap_prev[g], 0, S->jPrev + (int64_t)g * C.jmax, C.jmax, 0, 0};
-    const bool ok = ms_contour(f, idl, (uint32_t)g, o);
-    if (o.status) set_status(S, o.status);
-    if (!ok) {
-        C.state[g] = G_VANISHED;
-        S->cn_prev[g] = 0;
-        S->jn_prev[g] = 0;
-        C.volume[g] = 0;
-        return;
-    }
-    project_junctions(o.pts, o.n, o.js, o.jn);
-    S->cn_prev[g] = o.n;
-    S->jn_prev[g] = o.jn;
-    C.volume[g] = contour_volume(o.pts, o.n, C.h);
-}
-
 // ---------------------------------------------------------------------------
 // Initialisation for contour input (LSbox::calculateDistanceFunction,
 // src/box.cpp:342-400): every pixel (i, j) of the grain's box, at domain

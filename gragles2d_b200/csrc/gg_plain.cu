@@ -213,6 +213,11 @@ cudaError_t launch_convolution_plain(const NetConst& C, NetState* dS, cudaStream
     return cudaGetLastError();
 }
 
+void launch_levelset_plain(const NetConst& C, NetState* dS, cudaStream_t s) {
+    k_levelset_big<double><<<C.N, 32, 0, s>>>(C, dS);
+    k_levelset_w<double><<<(C.N + kGrainsPerBlock - 1) / kGrainsPerBlock, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
+}
+
 void launch_redistance_plain(const NetConst& C, NetState* dS, cudaStream_t s) {
     k_redistance<double, true><<<C.N, redist_threads<double, true>(), redist_smem<double, true>(), s>>>(C, dS);
     k_redistance<double, false><<<C.N, kRedistThreads, redist_smem<double, false>(), s>>>(C, dS);
@@ -229,8 +234,8 @@ cudaError_t plain_init(const NetConst& C, NetState* dS, const int32_t* d_ids, cu
     k_init_phi<double><<<C.N, 256, 0, s>>>(C, dS, d_ids);
     launch_redistance_plain(C, dS, s);
     k_swap_phi<<<1, 1, 0, s>>>(dS);
-    const int gt = 64;
-    k_init_contour<double><<<(C.N + gt - 1) / gt, gt, 0, s>>>(C, dS);
+    k_init_contour_big<double><<<C.N, 32, 0, s>>>(C, dS);
+    k_init_contour_w<double><<<(C.N + kGrainsPerBlock - 1) / kGrainsPerBlock, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
     return cudaGetLastError();
 }
 
@@ -261,7 +266,7 @@ cudaError_t plain_stage_kernel(const NetConst& C, NetState* dS, int which, cudaS
             break;
         case 2: k_second_order_w<<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS); break;
         case 3: k_compare<double><<<C.N, cfg.compare_threads, 0, s>>>(C, dS); break;
-        case 4: k_levelset_w<double><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS); break;
+        case 4: launch_levelset_plain(C, dS, s); break;
         case 5: k_alloc<<<1, 1024, 0, s>>>(C, dS, 2); break;
         case 6: k_neighbours_w<double><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS, reinterpret_cast<PointInfo*>(C.ptinfo)); break;
         case 7: launch_redistance_plain(C, dS, s); break;
@@ -294,7 +299,7 @@ cudaError_t plain_stages(const NetConst& C, NetState* dS, int stages, cudaStream
         if (tan) k_compare_t<<<C.N, 256, 0, s>>>(C, dS);
     }
     if (stages & ST_LEVELSET) {
-        k_levelset_w<double><<<wblocks, 32 * kGrainsPerBlock, 0, s>>>(C, dS);
+        launch_levelset_plain(C, dS, s);
         if (tan) k_area_t<<<(C.N + 3) / 4, 128, 0, s>>>(C, dS);  // warp per grain
     }
     if (stages & ST_REDIST) {

@@ -353,19 +353,28 @@ __device__ __forceinline__ double form_perimeter(const double2* P, int n, double
     else return perimeter_xy(P, n, h);
 }
 
+// LSbox::clearContourGrainArea (src/box.cpp:1888-1906) by the whole warp (every
+// pixel's test and write are its own).
 template <typename R>
 __device__ bool clear_area_xy(R* phi, const Box& b, const double2* P, int n, double h) {
     if (n == 0) return true;
+    const int lane = threadIdx.x & 31;
     double minx = P[0].x, maxx = P[0].x, miny = P[0].y, maxy = P[0].y;
-    for (int i = 0; i < n; i++) {
+    for (int i = lane; i < n; i += 32) {
         minx = fmin(minx, P[i].x);
         maxx = fmax(maxx, P[i].x);
         miny = fmin(miny, P[i].y);
         maxy = fmax(maxy, P[i].y);
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        minx = fmin(minx, __shfl_xor_sync(0xffffffffu, minx, o));
+        maxx = fmax(maxx, __shfl_xor_sync(0xffffffffu, maxx, o));
+        miny = fmin(miny, __shfl_xor_sync(0xffffffffu, miny, o));
+        maxy = fmax(maxy, __shfl_xor_sync(0xffffffffu, maxy, o));
+    }
     bool ok = true;
     for (int i = (int)(miny - 1); i < maxy + 1; i++)
-        for (int j = (int)(minx - 1); j < maxx + 1; j++) {
+        for (int j = (int)(minx - 1) + lane; j < maxx + 1; j += 32) {
             uint32_t k;
             if (!buf_index(b, i, j, &k)) {
                 ok = false;
@@ -373,26 +382,46 @@ __device__ bool clear_area_xy(R* phi, const Box& b, const double2* P, int n, dou
             }
             if ((double)phi[k] >= 0) phi[k] = (R)(-h);
         }
-    return ok;
+    return __all_sync(0xffffffffu, ok);
 }
 
-constexpr int kWalkPts = 448;  // shared-memory contour buffer per warp
-struct WalkShared;
-template <typename R>
-__device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint32_t own, ContourOut& o, int lane,
-                                   double2* xy, WalkShared& ws);
+// Shared buffers of one warp's contour extraction: the padded bitmap of the
+// box, the recorded walk steps, the contour points.  Boxes up to about 94 cells
+// take the small ones, four warps to a CTA; larger ones (to 222 cells) a CTA of
+// one warp with the large ones, beside them.  What fits neither is walked by one
+// lane in device memory, which takes some 250 us for a box of 100 cells.
+template <int kBitmapWords, int kSteps, int kPoints>
+struct WalkBuffers {
+    static constexpr int kBitmap = kBitmapWords, kTrace = kSteps, kPts = kPoints;
+    double2 xy[kPoints];
+    uint32_t bm[kBitmapWords];
+    uint16_t trace[kSteps];
+};
+using SmallWalk = WalkBuffers<400, 768, 448>;
+using LargeWalk = WalkBuffers<1570, 2048, 1024>;
+
+// Whether a box's padded bitmap fits.
+template <class W>
+__device__ __forceinline__ bool walk_fits(const Box& b) {
+    const int w = box_w(b), hgt = box_h(b), wpr = (w + 2 + 31) >> 5;
+    return w + 2 <= 1024 && (hgt + 2) * wpr + 1 <= W::kBitmap && (hgt + 1) * (w + 1) <= 65535;
+}
+
+template <class W, typename R>
+__device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint32_t own, ContourOut& o, int lane, W& ws);
 
 // Contour + junctions of one grain by one warp; returns false if no pixel
 // has phi >= 0.  The walk writes into the warp's shared buffer xy (or, for a
 // contour longer than the buffer, directly into the global contour);
 // junctions are projected one lane per junction.  On return *in_shared says
 // where the points are.
-template <typename R>
-__device__ bool extract_warp(const Field<R>& f, const uint32_t* idl, uint32_t own, ContourOut& o, int lane,
-                             double2* xy, bool* in_shared, WalkShared* ws) {
-    if (ws) {
+template <class W, typename R>
+__device__ bool extract_warp(const Field<R>& f, const uint32_t* idl, uint32_t own, ContourOut& o, int lane, W& ws,
+                             bool* in_shared) {
+    double2* const xy = ws.xy;
+    {
         const uint32_t st0 = o.status;
-        const int r = extract_bitmap_warp(f, idl, own, o, lane, xy, *ws);
+        const int r = extract_bitmap_warp(f, idl, own, o, lane, ws);
         if (r >= 0) {
             *in_shared = true;
             return r == 1;
@@ -410,9 +439,9 @@ __device__ bool extract_warp(const Field<R>& f, const uint32_t* idl, uint32_t ow
     const int gcap = o.cap;
     bool shared = true;
     if (lane == 0) {
-        o.cap = gcap < kWalkPts ? gcap : kWalkPts;
+        o.cap = gcap < W::kPts ? gcap : W::kPts;
         ms_walk(f, idl, own, f.b.x0 + start % w, f.b.y0 + start / w, o, xy);
-        if ((o.status & S_CONTOUR_OVERFLOW) && gcap > kWalkPts) {  // long contour: walk again into global memory
+        if ((o.status & S_CONTOUR_OVERFLOW) && gcap > W::kPts) {  // long contour: walk again into global memory
             o.status &= ~S_CONTOUR_OVERFLOW;
             o.cap = gcap;
             ms_walk(f, idl, own, f.b.x0 + start % w, f.b.y0 + start / w, o, (double2*)nullptr);
@@ -457,14 +486,6 @@ __device__ bool extract_warp(const Field<R>& f, const uint32_t* idl, uint32_t ow
     return true;
 }
 
-constexpr int kBitmapCap = 400;  // words of the padded bitmap (boxes up to about 94 x 94)
-constexpr int kTrace = 768;      // walk steps recorded per warp
-
-struct WalkShared {
-    uint32_t bm[kBitmapCap];
-    uint16_t trace[kTrace];
-};
-
 // Corner mask of the marching-squares cell whose top-left pixel is at padded
 // row tr, padded column lc (C_TL | C_TR from row tr, C_BL | C_BR from tr + 1).
 __device__ __forceinline__ int cell_mask(const uint32_t* bm, int wpr, int tr, int lc) {
@@ -497,14 +518,15 @@ constexpr uint32_t kMsEmit = 0xFFFFu & ~((1u << 0) | (1u << 6) | (1u << 9) | (1u
 // across the lanes in walk order.  Returns 0 if no pixel is inside, 1 on
 // success, -1 if the box or the walk does not fit the shared buffers (the
 // caller then walks in global memory).
-template <typename R>
+template <class W, typename R>
 __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint32_t own, ContourOut& o, int lane,
-                                   double2* xy, WalkShared& ws) {
+                                   W& ws) {
+    double2* const xy = ws.xy;
     const Box b = f.b;
     const int w = box_w(b), hgt = box_h(b);
     // padded bitmap: row r + 1, bit c + 1 hold pixel (r, c) of the box
     const int wpr = (w + 2 + 31) >> 5;
-    if (w + 2 > 1024 || (hgt + 2) * wpr + 1 > kBitmapCap) return -1;
+    if (!walk_fits<W>(b)) return -1;
     bool nonfinite = false;  // a NaN or infinity anywhere in the field
     for (int r0 = 0; r0 < hgt + 2; r0 += 8)  // eight rows of two words: 16 loads in flight
         for (int q0 = 0; q0 < wpr; q0 += 2) {
@@ -558,7 +580,6 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
     // direction is recovered later from the next recorded cell).  The switch
     // of the reference is evaluated as selects, so a step has no branch.
     const int cw = w + 1;
-    if ((hgt + 1) * cw > 65535) return -1;
     int nsteps = 0;
     uint32_t st = 0;
     if (lane == 0) {
@@ -577,10 +598,10 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
             lc += (next == MS_RIGHT) - (next == MS_LEFT);
             tr += (next == MS_DOWN) - (next == MS_UP);
             prev = next;
-            if (nsteps >= kTrace || nsteps > limit) break;
+            if (nsteps >= W::kTrace || nsteps > limit) break;
         } while (lc != lc_end || tr != tr_end);
         if (lc != lc_end || tr != tr_end) {
-            if (nsteps >= kTrace)
+            if (nsteps >= W::kTrace)
                 nsteps = -1;  // longer than the trace buffer: walk again in global memory
             else
                 st |= S_WALK_LIMIT;
@@ -679,7 +700,7 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
             const uint32_t eb = __ballot_sync(0xffffffffu, emit[k]);
             if (emit[k]) {
                 const int pos = ne + __popc(eb & lt);
-                if (pos < kWalkPts)
+                if (pos < W::kPts)
                     xy[pos] = make_double2(px, py);
                 else
                     point_overflow = true;
@@ -722,9 +743,9 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
         n += __popc(kb);
         __syncwarp();
     }
-    const int cap = o.cap < kWalkPts ? o.cap : kWalkPts;
+    const int cap = o.cap < W::kPts ? o.cap : W::kPts;
     if (n > 0 && (xy[0].x != xy[n - 1].x || xy[0].y != xy[n - 1].y)) {  // close the loop
-        if (lane == 0 && n < kWalkPts) xy[n] = xy[0];
+        if (lane == 0 && n < W::kPts) xy[n] = xy[0];
         n++;
     }
     if (n > cap) {
@@ -751,15 +772,9 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
 
 // grainhdl::level_set -> LSbox::extractContour (src/grainhdl.cpp:830-848,
 // src/box.cpp:1089-1153), one warp per grain.
-template <typename R>
-__global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_levelset_w(NetConst C, NetState* S) {
-    __shared__ double2 s_xy[kGrainsPerBlock][kWalkPts];
-    __shared__ WalkShared s_walk[kGrainsPerBlock];
+template <typename R, class W>
+__device__ __forceinline__ void levelset_grain(const NetConst& C, NetState* S, int g, W& walk) {
     const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    const int slot = blockIdx.x * kGrainsPerBlock + wid;
-    const int g = slot < C.N ? grain_at(S, slot) : C.N + 1;
-    if (g > C.N || halted(S)) return;
     const int st = C.state[g];
     const Box bc = S->box_cur[g];
     if (st != G_EXISTS) {
@@ -774,14 +789,14 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_levelset_w(NetConst
         }
         return;
     }
-    double2* xy = s_xy[wid];
+    double2* const xy = walk.xy;
     const int old_len = S->cn_prev[g];
     R* phi = phiA_of<R>(S) + S->off_cur[g];
     Field<R> f{phi, bc};
     const uint32_t* idl = S->idCur + S->off_cur[g];
     ContourOut o{S->contCur + S->coff_cur[g], S->ccap_cur[g], 0, S->jCur + (int64_t)g * C.jmax, C.jmax, 0, 0};
     bool shared = true;
-    bool ok = extract_warp(f, idl, (uint32_t)g, o, lane, xy, &shared, &s_walk[wid]);
+    bool ok = extract_warp(f, idl, (uint32_t)g, o, lane, walk, &shared);
     int irregular = 0;
     if (ok) {
         double newVolume = 0;
@@ -794,13 +809,14 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_levelset_w(NetConst
         regular_motion = __shfl_sync(0xffffffffu, regular_motion, 0);
         int tries = 0;
         while (!regular_motion) {  // clear the grain area and extract again (src/box.cpp:1099-1114)
-            if (lane == 0) {
-                const bool in_range = shared ? clear_area_xy(phi, bc, xy, o.n, C.h)
-                                             : clear_contour_area(phi, bc, o.pts, o.n, C.h);
-                if (!in_range) o.status |= S_INDEX;
-            }
+            bool in_range = true;
+            if (shared)
+                in_range = clear_area_xy(phi, bc, xy, o.n, C.h);
+            else if (lane == 0)
+                in_range = clear_contour_area(phi, bc, o.pts, o.n, C.h);
+            if (!in_range) o.status |= S_INDEX;
             __syncwarp();
-            ok = extract_warp(f, idl, (uint32_t)g, o, lane, xy, &shared, &s_walk[wid]);
+            ok = extract_warp(f, idl, (uint32_t)g, o, lane, walk, &shared);
             if (!ok) break;
             if (shared) newVolume = form_volume<R>(xy, o.n, C.h);
             if (lane == 0) {
@@ -854,26 +870,50 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_levelset_w(NetConst
     S->jn_cur[g] = o.jn;
 }
 
-// Initial contours of a voxelized network (distanceInitialisation ->
-// LSbox::extractContour on the initial distance field, as k_init_contour
-// does one thread per grain): one warp per grain with the level set's
-// warp-parallel extraction (bitmap walk, points, junctions and their
-// projection across the lanes), into the previous-step roles the first
-// corrector reads.
 template <typename R>
-__global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_init_contour_w(NetConst C, NetState* S) {
-    __shared__ double2 s_xy[kGrainsPerBlock][kWalkPts];
-    __shared__ WalkShared s_walk[kGrainsPerBlock];
-    const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_levelset_w(NetConst C, NetState* S) {
+    __shared__ SmallWalk s_walk[kGrainsPerBlock];
     const int wid = threadIdx.x >> 5;
-    const int g = blockIdx.x * kGrainsPerBlock + wid + 1;
-    if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
-    double2* xy = s_xy[wid];
+    const int slot = blockIdx.x * kGrainsPerBlock + wid;
+    const int g = slot < C.N ? grain_at(S, slot) : C.N + 1;
+    if (g > C.N || halted(S)) return;
+    if (C.state[g] == G_EXISTS && !walk_fits<SmallWalk>(S->box_cur[g])) return;  // k_levelset_big's
+    levelset_grain<R>(C, S, g, s_walk[wid]);
+}
+
+// The existing grains whose boxes do not fit the small buffers: one-warp CTAs
+// over all slots (which the work queue, where there is one, orders by
+// descending edge, so that they end at the first existing grain that fits).
+template <typename R>
+__global__ void __launch_bounds__(32) k_levelset_big(NetConst C, NetState* S) {
+    __shared__ LargeWalk s_walk;
+    if (halted(S)) return;
+    for (int slot = blockIdx.x; slot < C.N; slot += gridDim.x) {
+        const int g = grain_at(S, slot);
+        if (C.state[g] != G_EXISTS) continue;  // keeps its place in the queue
+        if (walk_fits<SmallWalk>(S->box_cur[g])) {
+            if (S->order) return;
+            continue;
+        }
+        levelset_grain<R>(C, S, g, s_walk);
+        __syncwarp();
+    }
+}
+
+// Initial contours of a voxelized network (distanceInitialisation ->
+// LSbox::extractContour on the initial distance field): one warp per grain
+// with the level set's warp-parallel extraction (bitmap walk, points, junctions
+// and their projection across the lanes), into the previous-step roles the
+// first corrector reads.
+template <typename R, class W>
+__device__ __forceinline__ void init_contour_grain(const NetConst& C, NetState* S, int g, W& walk) {
+    const int lane = threadIdx.x & 31;
+    double2* const xy = walk.xy;
     Field<R> f{phiA_of<R>(S) + S->off_cur[g], S->box_cur[g]};
     const uint32_t* idl = S->idPrev + S->off_prev[g];
     ContourOut o{S->contPrev + S->coff_prev[g], S->ccap_prev[g], 0, S->jPrev + (int64_t)g * C.jmax, C.jmax, 0, 0};
     bool shared = true;
-    const bool ok = extract_warp(f, idl, (uint32_t)g, o, lane, xy, &shared, &s_walk[wid]);
+    const bool ok = extract_warp(f, idl, (uint32_t)g, o, lane, walk, &shared);
     double vol = 0;
     if (ok && shared) {
         for (int i = lane; i < o.n; i += 32) {
@@ -899,6 +939,23 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_init_contour_w(NetC
     S->cn_prev[g] = o.n;
     S->jn_prev[g] = o.jn;
     C.volume[g] = vol;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_init_contour_w(NetConst C, NetState* S) {
+    __shared__ SmallWalk s_walk[kGrainsPerBlock];
+    const int wid = threadIdx.x >> 5;
+    const int g = blockIdx.x * kGrainsPerBlock + wid + 1;
+    if (g > C.N || C.state[g] != G_EXISTS || halted(S) || !walk_fits<SmallWalk>(S->box_cur[g])) return;
+    init_contour_grain<R>(C, S, g, s_walk[wid]);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(32) k_init_contour_big(NetConst C, NetState* S) {
+    __shared__ LargeWalk s_walk;
+    const int g = blockIdx.x + 1;
+    if (g > C.N || C.state[g] != G_EXISTS || halted(S) || walk_fits<SmallWalk>(S->box_cur[g])) return;
+    init_contour_grain<R>(C, S, g, s_walk);
 }
 
 // Per contour point result of the neighbour probe of buildDirectNeighbours.
