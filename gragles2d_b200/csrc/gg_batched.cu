@@ -847,9 +847,10 @@ cudaError_t batched_stages(const NetConst& C, NetState* dS, int stages, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, cudaStream_t s2, cudaStream_t s3,
-                               cudaEvent_t* ev, const LaunchCfg& cfg) {
+cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, const LaunchCfg& cfg) {
     if (C.N <= 0) return cudaSuccess;
+    const cudaStream_t s2 = cfg.side[0], s3 = cfg.side[1];
+    cudaEvent_t* const ev = cfg.ev;
     const int wblocks = (C.N + kGrainsPerBlock - 1) / kGrainsPerBlock;
     cudaError_t e;
     // second-order lists (lists and boxes only) beside convolution + corrector (fields)

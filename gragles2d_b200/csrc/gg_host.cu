@@ -64,6 +64,68 @@ void pinned_give(void* p, size_t bytes) {
     g_pinned_free.push_back(DevBuf{p, bytes});
 }
 
+// The streams and events of a context, kept by the process for its next
+// contexts in the same way (creating and destroying them cost 0.4 ms of a small
+// network's 9): taken for a device, given back with all their work done, at most
+// kStreamSets of them idle.
+struct StreamSet {
+    int device = -1;
+    cudaStream_t stream[3] = {};
+    cudaEvent_t timed[2] = {};
+    cudaEvent_t fork[kStepForks + 1] = {};  // the last one for the statistics read-back
+};
+constexpr size_t kStreamSets = 16;
+std::mutex g_streams_mutex;
+std::vector<StreamSet> g_streams_free;
+
+void streams_destroy(StreamSet& q) {
+    for (cudaEvent_t e : q.fork)
+        if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : q.timed)
+        if (e) cudaEventDestroy(e);
+    for (cudaStream_t t : q.stream)
+        if (t) cudaStreamDestroy(t);
+    q = StreamSet{};
+}
+
+// The current device must be `device`.
+cudaError_t streams_take(int device, StreamSet* out) {
+    {
+        std::lock_guard<std::mutex> lock(g_streams_mutex);
+        for (size_t i = 0; i < g_streams_free.size(); ++i)
+            if (g_streams_free[i].device == device) {
+                *out = g_streams_free[i];
+                g_streams_free.erase(g_streams_free.begin() + i);
+                return cudaSuccess;
+            }
+    }
+    StreamSet q;
+    q.device = device;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = cudaStreamCreateWithFlags(&q.stream[k], cudaStreamNonBlocking);
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreate(&q.timed[k]);
+    for (int k = 0; k < kStepForks + 1 && e == cudaSuccess; ++k)
+        e = cudaEventCreateWithFlags(&q.fork[k], cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        streams_destroy(q);
+        return e;
+    }
+    *out = q;
+    return cudaSuccess;
+}
+
+void streams_give(StreamSet& q) {
+    {
+        std::lock_guard<std::mutex> lock(g_streams_mutex);
+        if (g_streams_free.size() < kStreamSets) {
+            g_streams_free.push_back(q);
+            q = StreamSet{};
+            return;
+        }
+    }
+    streams_destroy(q);
+}
+
 }  // namespace
 
 struct gg_ctx {
@@ -115,34 +177,28 @@ struct gg_ctx {
     bool stats_wanted = false;
     bool stats_fresh = false;
     uint32_t* h_status = nullptr;
-    cudaEvent_t ev_done = nullptr;
     LaunchCfg cfg{256, 64, {nullptr, nullptr}, nullptr};
 
     cudaGraphExec_t graph = nullptr;
     bool sectors_stale = false;    // batched form: the corrector's sectors need a rebuild before the next step
     int32_t graph_kernels = 0;     // kernel nodes of the captured step graph
     int64_t kernel_launches = 0;   // graph_kernels per replay, summed
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaStream_t stream2 = nullptr, stream3 = nullptr;  // further branches of the captured batched step
-    cudaEvent_t fork[kStepForks] = {};
+    StreamSet set;                   // stream and the further ones of the captured batched step, events
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_done = nullptr;
     double last_ms = 0;
 
     ~gg_ctx() {
         if (graph) cudaGraphExecDestroy(graph);
-        if (stream) {
-            for (void* p : allocs) cudaFreeAsync(p, stream);  // back to the library's pool
-            cudaStreamSynchronize(stream);
-        }
+        if (!stream) return;
+        for (void* p : allocs) cudaFreeAsync(p, stream);  // back to the library's pool
+        bool idle = true;  // the side streams' work is joined into the first one's
+        for (cudaStream_t t : set.stream) idle = cudaStreamSynchronize(t) == cudaSuccess && idle;
         pinned_give(h_stats, h_stats_bytes);  // to the process's pinned buffers
         pinned_give(h_status, sizeof(uint32_t));
-        if (ev_done) cudaEventDestroy(ev_done);
-        if (ev0) cudaEventDestroy(ev0);
-        if (ev1) cudaEventDestroy(ev1);
-        for (cudaEvent_t e : fork)
-            if (e) cudaEventDestroy(e);
-        if (stream2) cudaStreamDestroy(stream2);
-        if (stream3) cudaStreamDestroy(stream3);
-        if (stream) cudaStreamDestroy(stream);
+        if (idle)
+            streams_give(set);
+        else
+            streams_destroy(set);
     }
 };
 
@@ -214,6 +270,52 @@ int dalloc(gg_ctx* c, T** out, size_t count, bool zero = true) {
     *out = reinterpret_cast<T*>(p);
     return GG_OK;
 }
+
+// Device arrays that are allocated together: the small ones share one block
+// for those to be zero-filled and one for the others (see dalloc), instead of an
+// allocation and a fill each (some 60 of them, 0.2 ms); arrays above 4 MiB stay
+// on their own, so that the pool can give them out again for another network's
+// sizes.  The pointers are set by commit().
+struct DeviceArrays {
+    struct Item {
+        void** out;
+        size_t bytes;
+        bool zero;
+    };
+    static constexpr size_t kShared = 4 << 20;
+    std::vector<Item> items;
+    template <typename T>
+    void add(T** out, size_t count, bool zero = true) {
+        items.push_back(Item{reinterpret_cast<void**>(out), sizeof(T) * (count > 0 ? count : 1), zero});
+    }
+    int commit(gg_ctx* c) {
+        for (const bool zero : {true, false}) {
+            size_t total = 0;
+            for (const Item& i : items) {
+                if (i.zero != zero) continue;
+                if (i.bytes <= kShared) {
+                    total += (i.bytes + 255) & ~(size_t)255;
+                } else {
+                    char* own = nullptr;
+                    const int rc = dalloc(c, &own, i.bytes, zero);
+                    if (rc) return rc;
+                    *i.out = own;
+                }
+            }
+            if (!total) continue;
+            char* base = nullptr;
+            const int rc = dalloc(c, &base, total, zero);
+            if (rc) return rc;
+            for (const Item& i : items)
+                if (i.zero == zero && i.bytes <= kShared) {
+                    *i.out = base;
+                    base += (i.bytes + 255) & ~(size_t)255;
+                }
+        }
+        items.clear();
+        return GG_OK;
+    }
+};
 
 std::string trim(const std::string& s) {
     size_t a = s.find_first_not_of(" \t\r\n");
@@ -559,6 +661,33 @@ std::mutex g_table_mutex;
 std::map<TableKey, std::vector<double>> g_gk_cache;
 std::map<TableKey, std::vector<float>> g_ck_cache;
 
+// Twiddles of every edge up to tmax, one after the other.  They depend on the
+// edge alone, so those of ordinary boxes (at most kTwiddleEdge: 1 MB) are
+// computed once per process, as far as any context needed them (0.5 ms for the
+// 160 edges of a small network).
+constexpr int kTwiddleEdge = 256;
+
+void twiddle_tables(int tmax, std::vector<double>& tw) {
+    static std::mutex mutex;
+    static std::vector<double> kept;  // edges 1 .. done
+    static int done = 0;
+    const auto append = [](int n, std::vector<double>& to) {
+        for (int k = 0; k < n; ++k) {
+            double re, im;
+            twiddle(n, k, &re, &im);
+            to.push_back(re);
+            to.push_back(im);
+        }
+    };
+    const int known = std::min(tmax, kTwiddleEdge);
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        for (; done < known; ++done) append(done + 1, kept);
+        tw.assign(kept.begin(), kept.begin() + (size_t)known * (known + 1));
+    }
+    for (int n = known + 1; n <= tmax; ++n) append(n, tw);
+}
+
 TableKey table_key(const gg_ctx* c, int n) {
     uint64_t bits;
     std::memcpy(&bits, &c->dt, sizeof bits);
@@ -827,15 +956,14 @@ int gg_create(const gg_params* p, int device, gg_ctx** out) {
         *out = c;
         return GG_E_CUDA;
     }
-    e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking);
-    for (int k = 0; k < kStepForks && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&c->fork[k], cudaEventDisableTiming);
-    c->cfg.side[0] = c->stream2;
-    c->cfg.side[1] = c->stream3;
-    c->cfg.ev = c->fork;
+    e = streams_take(device, &c->set);
+    c->stream = c->set.stream[0];
+    c->ev0 = c->set.timed[0];
+    c->ev1 = c->set.timed[1];
+    c->ev_done = c->set.fork[kStepForks];
+    c->cfg.side[0] = c->set.stream[1];
+    c->cfg.side[1] = c->set.stream[2];
+    c->cfg.ev = c->set.fork;
     if (e != cudaSuccess) {
         c->err = std::string("stream/event: ") + cudaGetErrorString(e);
         *out = c;
@@ -1307,10 +1435,9 @@ int gg_distance_initialisation(gg_ctx* c) {
     C.m_hagb = P.m_hagb;
 
     int rc;
-#define ALLOC(ptr, cnt) \
-    if ((rc = dalloc(c, &(ptr), (cnt))) != GG_OK) return rc
-#define ALLOC_UNZEROED(ptr, cnt) \
-    if ((rc = dalloc(c, &(ptr), (cnt), false)) != GG_OK) return rc
+    DeviceArrays arrays;
+#define ALLOC(ptr, cnt) arrays.add(&(ptr), (cnt))
+#define ALLOC_UNZEROED(ptr, cnt) arrays.add(&(ptr), (cnt), false)
     ALLOC(C.state, N + 1);
     ALLOC(C.regular, N + 1);
     ALLOC(C.inter_bnd, N + 1);
@@ -1330,8 +1457,6 @@ int gg_distance_initialisation(gg_ctx* c) {
     C.time_slope = P.time_slope;
     if (P.use_stored_elastic_energy) ALLOC(C.stored, N + 1);
     if (P.use_magnetic_field) ALLOC(C.magnetic, N + 1);
-    GG_CUDA(c, cudaMemsetAsync(C.gone_loop, 0xff, sizeof(int32_t) * (N + 1), c->stream));
-
     // tables: twiddles and Gaussian multipliers (plain), separable kernels (batched)
     std::vector<int64_t> tw_off(tmax + 1, 0), gk_off(tmax + 1, 0), ck_off(tmax + 1, 0);
     int64_t twn = 0, gkn = 0, ckn = 0;
@@ -1344,11 +1469,9 @@ int gg_distance_initialisation(gg_ctx* c) {
         ckn += n + 1;  // k_n, then its band radius
     }
     const bool plain = P.precision == GG_PRECISION_PLAIN;
-    std::vector<double> tw(plain ? 2 * twn : 2), gk(plain ? gkn : 1);
+    std::vector<double> tw(2), gk(plain ? gkn : 1);
     std::vector<float> ck(plain ? 1 : ckn);
-    if (plain)
-        for (int n = 1; n <= tmax; ++n)
-            for (int k = 0; k < n; ++k) twiddle(n, k, &tw[2 * (tw_off[n] + k)], &tw[2 * (tw_off[n] + k) + 1]);
+    if (plain) twiddle_tables(tmax, tw);  // at 2 tw_off[n]
     conv_tables(c, tmax, gk_off, ck_off, gk, ck);
     double* d_tw;
     double* d_gk;
@@ -1360,21 +1483,6 @@ int gg_distance_initialisation(gg_ctx* c) {
     ALLOC(d_twoff, tmax + 1);
     ALLOC(d_gkoff, tmax + 1);
     ALLOC(d_ckoff, tmax + 1);
-    GG_CUDA(c, cudaMemcpyAsync(d_tw, tw.data(), sizeof(double) * tw.size(), cudaMemcpyHostToDevice, c->stream));
-    GG_CUDA(c, cudaMemcpyAsync(d_gk, gk.data(), sizeof(double) * gk.size(), cudaMemcpyHostToDevice, c->stream));
-    GG_CUDA(c, cudaMemcpyAsync(d_ck, ck.data(), sizeof(float) * ck.size(), cudaMemcpyHostToDevice, c->stream));
-    GG_CUDA(c, cudaMemcpyAsync(d_twoff, tw_off.data(), sizeof(int64_t) * (tmax + 1), cudaMemcpyHostToDevice,
-                               c->stream));
-    GG_CUDA(c, cudaMemcpyAsync(d_gkoff, gk_off.data(), sizeof(int64_t) * (tmax + 1), cudaMemcpyHostToDevice,
-                               c->stream));
-    GG_CUDA(c, cudaMemcpyAsync(d_ckoff, ck_off.data(), sizeof(int64_t) * (tmax + 1), cudaMemcpyHostToDevice,
-                               c->stream));
-    C.tw = d_tw;
-    C.gk = d_gk;
-    C.ck = d_ck;
-    C.tw_off = d_twoff;
-    C.gk_off = d_gkoff;
-    C.ck_off = d_ckoff;
 
     // rotating state
     NetState& S = c->hS;
@@ -1391,68 +1499,34 @@ int gg_distance_initialisation(gg_ctx* c) {
         ALLOC(ccaps[k], N + 1);
     }
     for (int k = 0; k < 2; ++k) ALLOC(soffs[k], N + 1);
-    S.box_prev = boxes[0];
-    S.box_cur = boxes[1];
-    S.box_new = boxes[2];
-    S.off_prev = offs[0];
-    S.off_cur = offs[1];
-    S.off_new = offs[2];
-    S.soff_cur = soffs[0];
-    S.soff_new = soffs[1];
-    S.coff_prev = coffs[0];
-    S.coff_cur = coffs[1];
-    S.coff_new = coffs[2];
-    S.ccap_prev = ccaps[0];
-    S.ccap_cur = ccaps[1];
-    S.ccap_new = ccaps[2];
-    if (plain) {
-        double *pa, *pb, *sp_;
-        ALLOC(pa, phi_cap);
-        ALLOC(pb, phi_cap);
-        ALLOC(sp_, spec_cap);
-        S.phiA = pa;
-        S.phiB = pb;
-        S.spec = sp_;
-        if (c->tangents) {  // zero tangents: the initial field does not depend on the parameters
-            double *da, *db;
-            ALLOC(da, 4 * (size_t)phi_cap);
-            ALLOC(db, 4 * (size_t)phi_cap);
-            S.dphiA = da;
-            S.dphiB = db;
-            ALLOC(C.dvol, 4 * (size_t)(N + 1));
-            ALLOC(S.dcontPrev, 8 * (size_t)cont_cap);
-            ALLOC(S.dcontCur, 8 * (size_t)cont_cap);
-            ALLOC(C.dseg, 4 * (size_t)cont_cap);
-        }
-    } else {
-        float *pa, *pb, *sp_;
-        ALLOC_UNZEROED(pa, phi_cap);  // fields and the convolution's scratch: read only inside written boxes
-        ALLOC_UNZEROED(pb, phi_cap);
-        ALLOC_UNZEROED(sp_, spec_cap);
-        S.phiA = pa;
-        S.phiB = pb;
-        S.spec = sp_;
+    // the batched form's fields and the convolution's scratch are read only
+    // inside written boxes
+    arrays.add(reinterpret_cast<char**>(&S.phiA), rsz * (size_t)phi_cap, plain);
+    arrays.add(reinterpret_cast<char**>(&S.phiB), rsz * (size_t)phi_cap, plain);
+    arrays.add(reinterpret_cast<char**>(&S.spec), rsz * (size_t)spec_cap, plain);
+    if (plain && c->tangents) {  // zero tangents: the initial field does not depend on the parameters
+        arrays.add(reinterpret_cast<double**>(&S.dphiA), 4 * (size_t)phi_cap);
+        arrays.add(reinterpret_cast<double**>(&S.dphiB), 4 * (size_t)phi_cap);
+        ALLOC(C.dvol, 4 * (size_t)(N + 1));
+        ALLOC(S.dcontPrev, 8 * (size_t)cont_cap);
+        ALLOC(S.dcontCur, 8 * (size_t)cont_cap);
+        ALLOC(C.dseg, 4 * (size_t)cont_cap);
+    }
+    if (!plain) {
         ALLOC(C.segacc, cont_cap);
         c->sectors_stale = true;  // built one step ahead
     }
     if (!plain || !C.isotropic) {  // the corrector's sectors
-        char* pk;
-        ALLOC(pk, batched_sector_pack_bytes() * (size_t)(N + 1));
-        C.secpack = pk;
+        arrays.add(reinterpret_cast<char**>(&C.secpack), batched_sector_pack_bytes() * (size_t)(N + 1));
         ALLOC(C.segsec, cont_cap);
     }
     if (plain && !C.isotropic) ALLOC_UNZEROED(C.segacc64, cont_cap);
-    (void)rsz;
     ALLOC(S.idPrev, phi_cap);
     ALLOC(S.idCur, phi_cap);
     ALLOC_UNZEROED(S.contPrev, cont_cap);  // contour data: read up to the written counts
     ALLOC_UNZEROED(S.contCur, cont_cap);
     ALLOC_UNZEROED(S.segPrev, cont_cap);
-    {
-        double* pt;
-        ALLOC_UNZEROED(pt, 4 * (size_t)cont_cap);  // PointInfo: 32 bytes per contour point
-        C.ptinfo = pt;
-    }
+    arrays.add(reinterpret_cast<double**>(&C.ptinfo), 4 * (size_t)cont_cap, false);  // PointInfo: 32 bytes each
     ALLOC(S.cn_prev, N + 1);
     ALLOC(S.cn_cur, N + 1);
     ALLOC(S.jPrev, (size_t)C.jmax * (N + 1));
@@ -1470,6 +1544,37 @@ int gg_distance_initialisation(gg_ctx* c) {
 
 #undef ALLOC
 #undef ALLOC_UNZEROED
+    if ((rc = arrays.commit(c)) != GG_OK) return rc;
+    S.box_prev = boxes[0];
+    S.box_cur = boxes[1];
+    S.box_new = boxes[2];
+    S.off_prev = offs[0];
+    S.off_cur = offs[1];
+    S.off_new = offs[2];
+    S.soff_cur = soffs[0];
+    S.soff_new = soffs[1];
+    S.coff_prev = coffs[0];
+    S.coff_cur = coffs[1];
+    S.coff_new = coffs[2];
+    S.ccap_prev = ccaps[0];
+    S.ccap_cur = ccaps[1];
+    S.ccap_new = ccaps[2];
+    GG_CUDA(c, cudaMemsetAsync(C.gone_loop, 0xff, sizeof(int32_t) * (N + 1), c->stream));
+    GG_CUDA(c, cudaMemcpyAsync(d_tw, tw.data(), sizeof(double) * tw.size(), cudaMemcpyHostToDevice, c->stream));
+    GG_CUDA(c, cudaMemcpyAsync(d_gk, gk.data(), sizeof(double) * gk.size(), cudaMemcpyHostToDevice, c->stream));
+    GG_CUDA(c, cudaMemcpyAsync(d_ck, ck.data(), sizeof(float) * ck.size(), cudaMemcpyHostToDevice, c->stream));
+    GG_CUDA(c, cudaMemcpyAsync(d_twoff, tw_off.data(), sizeof(int64_t) * (tmax + 1), cudaMemcpyHostToDevice,
+                               c->stream));
+    GG_CUDA(c, cudaMemcpyAsync(d_gkoff, gk_off.data(), sizeof(int64_t) * (tmax + 1), cudaMemcpyHostToDevice,
+                               c->stream));
+    GG_CUDA(c, cudaMemcpyAsync(d_ckoff, ck_off.data(), sizeof(int64_t) * (tmax + 1), cudaMemcpyHostToDevice,
+                               c->stream));
+    C.tw = d_tw;
+    C.gk = d_gk;
+    C.ck = d_ck;
+    C.tw_off = d_twoff;
+    C.gk_off = d_gkoff;
+    C.ck_off = d_ckoff;
 
     // initial per-grain data
     const std::vector<double>& quat = c->quat;
@@ -1737,8 +1842,7 @@ int gg_step(gg_ctx* c, int32_t loop, int32_t nsteps) {
         if (!c->graph) {
             cudaGraph_t gr;
             GG_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = batched_step_graph(c->C, c->dS, c->stream, c->stream2, c->stream3, c->fork,
-                                               c->cfg);
+            cudaError_t e = batched_step_graph(c->C, c->dS, c->stream, c->cfg);
             cudaError_t e2 = cudaStreamEndCapture(c->stream, &gr);
             if (e != cudaSuccess) return cuda_fail(c, e, "capture");
             if (e2 != cudaSuccess) return cuda_fail(c, e2, "end capture");
@@ -1778,7 +1882,6 @@ int gg_step(gg_ctx* c, int32_t loop, int32_t nsteps) {
         // after the timed region: the statistics and the status word in one
         // pinned copy each, then one wait for all of it
         if (!c->h_status) GG_CUDA(c, pinned_take(reinterpret_cast<void**>(&c->h_status), sizeof(uint32_t)));
-        if (!c->ev_done) GG_CUDA(c, cudaEventCreateWithFlags(&c->ev_done, cudaEventDisableTiming));
         GG_CUDA(c, pack_stats(c->C, c->dS, c->d_stats, c->stream));
         GG_CUDA(c, cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(gg_grain_stats) * (size_t)c->N,
                                    cudaMemcpyDeviceToHost, c->stream));

@@ -37,10 +37,10 @@ cudaError_t plain_init_polygon(const NetConst& C, NetState* dS, cudaStream_t s);
 cudaError_t batched_stages(const NetConst& C, NetState* dS, int stages, cudaStream_t s, const LaunchCfg& cfg);
 // The whole batched step for graph capture on s, with the independent stages
 // (second-order lists beside convolution + corrector, volume / energy /
-// neighbours beside redistancing) forked onto s2 and s3 through the events ev.
+// neighbours beside redistancing) forked onto the side streams of cfg through
+// its events.
 constexpr int kStepForks = 6;
-cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, cudaStream_t s2, cudaStream_t s3,
-                               cudaEvent_t* ev, const LaunchCfg& cfg);
+cudaError_t batched_step_graph(const NetConst& C, NetState* dS, cudaStream_t s, const LaunchCfg& cfg);
 size_t conv_sep_smem(int tmax, int edge);
 cudaError_t batched_prepare(int tmax);
 cudaError_t batched_init(const NetConst& C, NetState* dS, const int32_t* d_ids, cudaStream_t s);
