@@ -216,10 +216,18 @@ size_t conv_sep_smem(int tmax, int edge) {
 // with the previous contour staged in shared memory (FP32 box-local
 // coordinates) and the per-pixel work in FP32, except the discrete decisions
 // of the projection, which follow the reference's FP64 arithmetic.  Each
-// warp takes one 8 x 4 tile of the box at a time.  The main kernel stages
-// contours up to kCorrStagedPts points; the large-contour kernel, persistent
-// over NetState::big_list, up to kCorrBigPts; longer ones are read from
-// device memory in FP64.
+// warp scans the box in tiles and collects the pixels near the boundary, about a
+// fifth, in a queue that full warps correct, each lane searching its own cell
+// window.  The main kernel stages contours up to kCorrStagedPts points; the
+// large-contour kernel, persistent over NetState::big_list, up to kCorrBigPts;
+// longer ones are read from device memory in FP64.
+//
+// 20,000 Read-Shockley grains: 973 us with a warp correcting the pixels of its
+// 8 x 4 tile in place (a third of the lanes busy, one pixel's loads in flight
+// per lane), 605 us with the queue, of which the set-up takes 120 (a chain of
+// dependent loads and five barriers), the scan 160 and the corrections 300;
+// their floor, two fields read and a little written, is 60.  What bounds it is
+// latency at 7 CTAs of 72 registers per SM (6: 676, 8 with spills: 676).
 constexpr int kCorrBigPts = 1024;
 
 // Packed FP32 pairs (sm_100 f32x2 arithmetic).
@@ -245,21 +253,22 @@ constexpr int kCellMax = 24;          // cells per side
 template <int kPts>  // vertices bucketed (the staged contours)
 struct VertexBuckets {
     int ncx, ncy, cell;
+    float inv;  // 1 / cell
     int end[kCellMax * kCellMax + 1];  // after the fill: end[c + 1] = first vertex of cell c
     short list[kPts];
 };
 
 template <int kPts>
-__device__ __forceinline__ int bucket_of(const VertexBuckets<kPts>& B, double lx, double ly) {
-    int cx = (int)floor(lx / B.cell), cy = (int)floor(ly / B.cell);
-    cx = cx < 0 ? 0 : (cx >= B.ncx ? B.ncx - 1 : cx);
-    cy = cy < 0 ? 0 : (cy >= B.ncy ? B.ncy - 1 : cy);
+__device__ __forceinline__ int bucket_of(const VertexBuckets<kPts>& B, float2 v) {
+    const int cx = min(max((int)floorf(v.x * B.inv), 0), B.ncx - 1);
+    const int cy = min(max((int)floorf(v.y * B.inv), 0), B.ncy - 1);
     return cy * B.ncx + cx;
 }
 
 // All threads: buckets of the vertices 0 .. npts-1 from their staged FP32
-// box-local coordinates P32 (each within 2^-24 L of the exact one, far inside
-// the search's 1e-3 cell margin).  Ends with a barrier.
+// box-local coordinates P32 (each within 2^-24 L of the exact one; the cell from
+// the product with 1 / cell adds 2^-23 L, all far inside the search's 1e-3
+// margin for the boxes of at most kPts vertices).  Ends with a barrier.
 template <int kPts>
 __device__ void build_buckets(VertexBuckets<kPts>& B, const float2* P32, int npts, int wi, int hi) {
     const int cs = max(4, (max(wi, hi) + kCellMax - 1) / kCellMax);
@@ -268,11 +277,12 @@ __device__ void build_buckets(VertexBuckets<kPts>& B, const float2* P32, int npt
         B.ncx = ncx;
         B.ncy = ncy;
         B.cell = cs;
+        B.inv = 1.f / (float)cs;
     }
     for (int c = threadIdx.x; c <= nc; c += blockDim.x) B.end[c] = 0;
     __syncthreads();
     for (int k = threadIdx.x; k < npts; k += blockDim.x)
-        atomicAdd(&B.end[bucket_of(B, (double)P32[k].x, (double)P32[k].y) + 1], 1);
+        atomicAdd(&B.end[bucket_of(B, P32[k]) + 1], 1);
     __syncthreads();
     if (threadIdx.x < 32) {  // inclusive scan of the counts by one warp
         int carry = 0;
@@ -289,7 +299,7 @@ __device__ void build_buckets(VertexBuckets<kPts>& B, const float2* P32, int npt
     }
     __syncthreads();
     for (int k = threadIdx.x; k < npts; k += blockDim.x) {
-        const int pos = atomicSub(&B.end[bucket_of(B, (double)P32[k].x, (double)P32[k].y) + 1], 1) - 1;
+        const int pos = atomicSub(&B.end[bucket_of(B, P32[k]) + 1], 1) - 1;
         B.list[pos] = (short)k;
     }
     __syncthreads();
@@ -299,50 +309,55 @@ constexpr unsigned kKeyIndexBits = 10;
 constexpr unsigned kKeyIndexMask = (1u << kKeyIndexBits) - 1u;
 static_assert(kCorrStagedPts <= kCorrBigPts && kCorrBigPts <= (1 << kKeyIndexBits), "vertex index must fit the key");
 
-// The reference's nearest vertex of the pixels (px, py) of the 32 lanes of a
-// warp (grid coordinates; all lanes call it, `need` lanes are the pixels
-// that want it).  The lanes scan together the vertices of the union of their
-// 3 x 3 cell windows in FP32 on the staged box-local contour P32 (each
-// coordinate within 2^-24 L of the exact local value, L the box edge, so a
-// squared distance d within 3 sqrt(d) 2^-24 L + 3e-7 d of the exact one):
-// each candidate is one 32-bit key, the distance's bits with the low 10
-// replaced by the vertex index, and a lane keeps its smallest key k1 and the
-// second smallest k2.  A lane whose two best lie within twice the rounding
-// bound (tie_margin with eps_c = 8 2^-24 L; the keys' truncation taken on
-// both sides) measures the candidates within that margin again in FP64 from
-// the contour itself, lowest index first at equal distance.  A lane whose
-// best distance exceeds (cell - 1e-3)^2 scans every vertex in FP64 (a vertex
-// within `cell` of the pixel lies in its window).
+// The reference's nearest vertex of the pixel (px, py) (grid coordinates), by
+// one lane.  It scans the vertices of its 3 x 3 cell window in FP32 on the
+// staged box-local contour P32 (each coordinate within 2^-24 L of the exact
+// local value, L the box edge, so a squared distance d within 3 sqrt(d) 2^-24 L
+// + 3e-7 d of the exact one): each candidate is one 32-bit key, the distance's
+// bits with the low 10 replaced by the vertex index, and the lane keeps its
+// smallest key k1 and the second smallest k2.  The window's three cell rows are
+// three ranges of the list, walked as one so that the warp's trip count is the
+// longest window and not the sum of the longest rows.  A lane whose two best lie
+// within twice the rounding bound (tie_margin with eps_c = 8 2^-24 L; the keys'
+// truncation taken on both sides) measures the candidates within that margin
+// again in FP64 from the contour itself, lowest index first at equal distance.
+// A lane whose best distance exceeds (cell - 1e-3)^2 scans every vertex in FP64
+// (a vertex within `cell` of the pixel lies in its window).
 template <int kPts>
-__device__ int nearest_vertex_warp(const VertexBuckets<kPts>& B, const float2* P32, const CPoint* P, int npts, int px,
-                                   int py, int ox, int oy, float eps_c, bool need) {
-    const unsigned FULL = 0xffffffffu;
+__device__ __forceinline__ int nearest_vertex(const VertexBuckets<kPts>& B, const float2* P32, const CPoint* P,
+                                              int npts, int px, int py, int ox, int oy, float eps_c) {
     const int cs = B.cell;
     const int lx = px - ox, ly = py - oy;
-    const int cx = min(max(lx / cs, 0), B.ncx - 1), cy = min(max(ly / cs, 0), B.ncy - 1);
-    const int ux0 = max(__reduce_min_sync(FULL, need ? cx : INT_MAX) - 1, 0);
-    const int ux1 = min(__reduce_max_sync(FULL, need ? cx : INT_MIN) + 1, B.ncx - 1);
-    const int uy0 = max(__reduce_min_sync(FULL, need ? cy : INT_MAX) - 1, 0);
-    const int uy1 = min(__reduce_max_sync(FULL, need ? cy : INT_MIN) + 1, B.ncy - 1);
     const float fx = (float)lx, fy = (float)ly;
-    unsigned k1 = 0xffffffffu, k2 = 0xffffffffu;
+    // the pixel's cell (half a pixel in, the rounding of 1 / cell is no matter)
+    const int cx = min(max((int)floorf((fx + 0.5f) * B.inv), 0), B.ncx - 1);
+    const int cy = min(max((int)floorf((fy + 0.5f) * B.inv), 0), B.ncy - 1);
     const int ncell = B.ncx * B.ncy;
-    for (int yy = uy0; yy <= uy1; ++yy) {
-        // cells ux0 .. ux1 of a row are consecutive in the list
-        const int q0 = B.end[yy * B.ncx + ux0 + 1];
-        const int cl = yy * B.ncx + ux1;
-        const int q1 = cl + 1 < ncell ? B.end[cl + 2] : npts;
-        for (int q = q0; q < q1; ++q) {
-            const int k = B.list[q];
-            const float2 v = P32[k];
-            const float dx = fx - v.x, dy = fy - v.y;
-            const float d = fmaf(dy, dy, dx * dx);
-            const unsigned key = (__float_as_uint(d) & ~kKeyIndexMask) | (unsigned)k;
-            k2 = min(k2, max(k1, key));
-            k1 = min(k1, key);
+    int start[3], upto[3], total = 0;
+    for (int r = 0; r < 3; ++r) {
+        const int yy = cy - 1 + r;
+        int q0 = 0, q1 = 0;
+        if (yy >= 0 && yy < B.ncy) {
+            // the cells of a row are consecutive in the list
+            q0 = B.end[yy * B.ncx + max(cx - 1, 0) + 1];
+            const int cl = yy * B.ncx + min(cx + 1, B.ncx - 1);
+            q1 = cl + 1 < ncell ? B.end[cl + 2] : npts;
         }
+        start[r] = q0 - total;
+        total += q1 - q0;
+        upto[r] = total;
     }
-    if (!need) return -1;
+    unsigned k1 = 0xffffffffu, k2 = 0xffffffffu;
+#pragma unroll 2
+    for (int q = 0; q < total; ++q) {
+        const int k = B.list[q + (q < upto[0] ? start[0] : q < upto[1] ? start[1] : start[2])];
+        const float2 v = P32[k];
+        const float dx = fx - v.x, dy = fy - v.y;
+        const float d = fmaf(dy, dy, dx * dx);
+        const unsigned key = (__float_as_uint(d) & ~kKeyIndexMask) | (unsigned)k;
+        k2 = min(k2, max(k1, key));
+        k1 = min(k1, key);
+    }
     const float d1 = __uint_as_float(min(k1 | kKeyIndexMask, 0x7f7fffffu));
     const float r = (float)cs - 1e-3f;
     const bool covered = k1 != 0xffffffffu && d1 <= r * r;
@@ -364,19 +379,14 @@ __device__ int nearest_vertex_warp(const VertexBuckets<kPts>& B, const float2* P
         const double dpx = (double)px, dpy = (double)py;
         double best = 1000000.0;
         nearest = -1;
-        for (int yy = max(cy - 1, 0); yy <= min(cy + 1, B.ncy - 1); ++yy) {
-            const int q0 = B.end[yy * B.ncx + max(cx - 1, 0) + 1];
-            const int cl = yy * B.ncx + min(cx + 1, B.ncx - 1);
-            const int q1 = cl + 1 < ncell ? B.end[cl + 2] : npts;
-            for (int q = q0; q < q1; ++q) {
-                const int k = B.list[q];
-                const float dx = fx - P32[k].x, dy = fy - P32[k].y;
-                if (fmaf(dy, dy, dx * dx) > thr) continue;
-                const double d = dist2_rn(dpx, dpy, P[k]);
-                if (d < best || (d == best && k < nearest)) {
-                    best = d;
-                    nearest = k;
-                }
+        for (int q = 0; q < total; ++q) {
+            const int k = B.list[q + (q < upto[0] ? start[0] : q < upto[1] ? start[1] : start[2])];
+            const float dx = fx - P32[k].x, dy = fy - P32[k].y;
+            if (fmaf(dy, dy, dx * dx) > thr) continue;
+            const double d = dist2_rn(dpx, dpy, P[k]);
+            if (d < best || (d == best && k < nearest)) {
+                best = d;
+                nearest = k;
             }
         }
     }
@@ -433,40 +443,43 @@ __device__ __forceinline__ int segment_step(const float2* P32, const CPoint* P, 
     return before ? nv - 1 : nearest;
 }
 
+// An interpolating sector as the per-pixel weights use it.
+struct SectorWeights {
+    float length, left_w, right_w, boundary_w;
+    int32_t both;  // boundary sectors on both sides
+};
+
 // Shared memory of one CTA of the batched corrector.
 template <int kPts>
 struct CorrectorSmem {
     float2 sp[kPts];  // the contour, FP32 box-local
     NbTable nbt;
     VertexBuckets<kPts> vb;
-    double cw[kMaxConstSectors];
-    InterpSector is[kMaxInterpSectors];
+    float cw[kMaxConstSectors];
+    SectorWeights is[kMaxInterpSectors];
     int16_t sid[kPts];  // per-segment sector table
     float acc[kPts];
+    unsigned queue[4][160];  // per warp: pixels to correct, y << 16 | x
 };
 
-// Whether grain g is corrected at all this step (uniform over the CTA).
-__device__ __forceinline__ bool corrects(const NetConst& C, const NetState* S, int g) {
-    return g <= C.N && C.state[g] == G_EXISTS && C.regular[g] != 0 && S->loop != 0 && !halted(S);
-}
-
-// The correction of grain g by the whole CTA (all threads call it; every
-// early return is uniform over the CTA).
+// The correction of grain g, if it is corrected at all this step, by the whole
+// CTA (all threads call it; every early return is uniform over the CTA).
 template <bool kForces, int kPts>
 __device__ __forceinline__ void correct_grain(const NetConst& C, NetState* S, int g, CorrectorSmem<kPts>& sm) {
     float2* sp = sm.sp;
     NbTable& nbt = sm.nbt;
     VertexBuckets<kPts>& vb = sm.vb;
-    double* s_cw = sm.cw;
-    InterpSector* s_is = sm.is;
     int16_t* s_sid = sm.sid;
     float* s_acc = sm.acc;
+    // everything that hangs on g alone is loaded before the first decision
+    const bool live = C.state[g] == G_EXISTS & C.regular[g] != 0 & S->loop != 0 & !halted(S);
     const int64_t coff = S->coff_prev[g];
-    const CPoint* P = S->contPrev + coff;
     const int size = S->cn_prev[g];
-    if (size < 2) return;
-    const Box ib = S->box_prev[g];
-    const uint32_t* idl = S->idPrev + S->off_prev[g];
+    const Box ib = S->box_prev[g], bo = S->box_cur[g];
+    const int64_t off_prev = S->off_prev[g], off_cur = S->off_cur[g];
+    if (!live || size < 2) return;
+    const CPoint* P = S->contPrev + coff;
+    const uint32_t* idl = S->idPrev + off_prev;
     const bool staged = size <= kPts;
     // the contour in FP32 coordinates local to the previous box (its points
     // lie inside it), so the search's rounding is relative to the box edge
@@ -477,8 +490,12 @@ __device__ __forceinline__ void correct_grain(const NetConst& C, NetState* S, in
     // the sectors, built one step ahead (k_sectors), and the per-segment table
     const SectorPack* pk = reinterpret_cast<const SectorPack*>(C.secpack) + g;
     const int nconst = pk->nconst, ninterp = pk->ninterp;
-    for (int c = threadIdx.x; c < nconst; c += blockDim.x) s_cw[c] = pk->cw[c];
-    for (int c = threadIdx.x; c < ninterp; c += blockDim.x) s_is[c] = pk->is[c];
+    for (int c = threadIdx.x; c < nconst; c += blockDim.x) sm.cw[c] = (float)pk->cw[c];
+    for (int c = threadIdx.x; c < ninterp; c += blockDim.x) {
+        const InterpSector& from = pk->is[c];
+        sm.is[c] = SectorWeights{(float)from.length, (float)from.left_w, (float)from.right_w, (float)from.boundary_w,
+                                 from.lb >= 0 && from.rb >= 0};
+    }
     const int16_t* tsid = C.segsec + coff;
     const float* tacc = C.segacc + coff;
     if (staged) {
@@ -486,128 +503,159 @@ __device__ __forceinline__ void correct_grain(const NetConst& C, NetState* S, in
             s_sid[q] = tsid[q];
             s_acc[q] = tacc[q];
         }
-        tsid = s_sid;
-        tacc = s_acc;
     }
     build_nb_table(C, g, nbt);
     if (staged) build_buckets(vb, sp, size - 1, box_w(ib), box_h(ib));  // ends with a barrier
     __syncthreads();
-    const Box bo = S->box_cur[g];
     const int x0 = ib.x0 < bo.x0 ? bo.x0 : ib.x0;
     const int y0 = ib.y0 < bo.y0 ? bo.y0 : ib.y0;
     const int x1 = ib.x1 > bo.x1 ? bo.x1 : ib.x1;
     const int y1 = ib.y1 > bo.y1 ? bo.y1 : ib.y1;
     if (x1 <= x0 || y1 <= y0) return;
     const int w = x1 - x0, hgt = y1 - y0;
-    const float* in = reinterpret_cast<const float*>(S->phiA) + S->off_cur[g];
-    float* out = reinterpret_cast<float*>(S->phiB) + S->off_cur[g];
+    const float* in = reinterpret_cast<const float*>(S->phiA) + off_cur;
+    float* out = reinterpret_cast<float*>(S->phiB) + off_cur;
     const int wo = box_w(bo), wi = box_w(ib);
     const float delta = (float)C.delta;
     const int real = size - 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int ntx = (w + 7) >> 3, ntiles = ntx * ((hgt + 3) >> 2);
-    uint32_t st = 0;
+    const int ntx = (w + 15) >> 4;
     const bool far_ok = C.gamma_hagb <= 1.0 && C.m_hagb <= 1.0;
+    // driving-force terms (src/box.cpp:511-527) of a pixel owned by `id`
+    const auto force = [&](uint32_t id) {
+        double f = 0;
+        if (C.stored) f += nb_stored_force(nbt, (int)id) * C.dt / C.time_slope;
+        if (C.magnetic) f += nb_magnetic_force(nbt, (int)id) * C.dt / C.time_slope;
+        return (float)f;
+    };
     // rounding margin of the FP32 segment step: 8 2^-24 L, L bounding every
     // local coordinate of the contour and the pixels
     const float eps_c = 8.f * 5.9604645e-8f * (float)(max(wi, box_h(ib)) + 2);
-    // one warp per 8 x 4 tile; pixels at or below -delta are set to -delta
-    for (int t = warp; t < ntiles; t += nwarps) {
-        const int x = (t % ntx) * 8 + (lane & 7), y = (t / ntx) * 4 + (lane >> 3);
-        const bool inside = x < w && y < hgt;
-        const int i = y0 + y, j = x0 + x;
-        const int k = (i - bo.y0) * wo + (j - bo.x0);
-        float val = 0.f, conv = 0.f;
-        uint32_t id = 0;
-        if (inside) {
-            val = __ldg(in + k);
-            conv = out[k];
-            id = idl[(i - ib.y0) * wi + (j - ib.x0)];
-        }
-        const bool valid = inside && val > -delta;
-        // driving-force terms (src/box.cpp:511-527) of inside pixels
-        float se = 0.f;
-        if (kForces && inside) {
-            double f = 0;
-            if (C.stored) f += nb_stored_force(nbt, (int)id) * C.dt / C.time_slope;
-            if (C.magnetic) f += nb_magnetic_force(nbt, (int)id) * C.dt / C.time_slope;
-            se = (float)f;
-        }
-        if (inside && !valid) out[k] = -delta - se;
-        // The corrected value val + (conv - val) w lies between val and
-        // 2 conv - val for every weight w in [0, 2]; with the relative
-        // high-angle energy and mobility at most 1 the weights (energy x
-        // mobility products, junction sums of three energies, their blends)
-        // stay below 2 (far_ok).  When val, conv and
-        // 2 conv - val all lie on the same side beyond 0.3 delta (2.1 cells),
-        // the pixel keeps that side whatever its weight, and it is not next to
-        // a sign change of these near-distance fields; only signs and the
-        // values next to sign changes reach the comparison's zero crossings
-        // and the redistancing that replaces the field.  Such a pixel takes
-        // weight 1 (the convolved value) without the projection.  (On the
-        // 20,000-grain workload the areas stay bit-identical for 10 steps and
-        // within 1.3e-7 relative, in 18 grains, after 40.)
-        const float far_level = 0.3f * delta, stretched = 2.f * conv - val;
-        const bool far = far_ok && valid &&
-                         ((val >= far_level && conv >= far_level && stretched >= far_level) ||
-                          (val <= -far_level && conv <= -far_level && stretched <= -far_level));
-        if (far) out[k] = conv - se;
-        const bool need = valid && !far;
-        if (__ballot_sync(0xffffffffu, need) == 0u) continue;
-        float lambda = 0.f;
-        int segment = 0;
-        if (staged) {
-            const int nv = nearest_vertex_warp(vb, sp, P, size - 1, j, i, ox, oy, eps_c, need);
-            if (!need) continue;
-            if (nv >= 0) segment = segment_step(sp, P, size, j, i, ox, oy, eps_c, nv, &lambda);
-        } else {
-            if (!need) continue;
-            double dl = 0;
-            segment = project_to_boundary(P, size, (double)j, (double)i, &dl);
-            lambda = (float)dl;
-        }
-        const int sid = tsid[segment];
-        float interpolator = sid <= -2 ? tacc[segment] : 0.f;
-        float weight;
-        if (sid >= 0) {
-            weight = (float)s_cw[sid];
-        } else if (sid == -1) {
-            // getGBEnergyTimesGBMobility(i, j) through the neighbour table
-            weight = 1.f;
-            for (int e = 0; e < nbt.n; ++e)
-                if (nbt.id[e] == (int)id) {
-                    weight = (float)nbt.w[e];
-                    break;
+    // Each warp scans 16 x 8 tiles, four pixels per lane with their loads in
+    // flight together: pixels at or below -delta are set to -delta, far ones
+    // keep their convolved value, and the others, about a fifth, join the warp's
+    // queue, which is corrected by full warps.
+    //
+    // The corrected value val + (conv - val) w lies between val and
+    // 2 conv - val for every weight w in [0, 2]; with the relative
+    // high-angle energy and mobility at most 1 the weights (energy x
+    // mobility products, junction sums of three energies, their blends)
+    // stay below 2 (far_ok).  When val, conv and
+    // 2 conv - val all lie on the same side beyond 0.3 delta (2.1 cells),
+    // the pixel keeps that side whatever its weight, and it is not next to
+    // a sign change of these near-distance fields; only signs and the
+    // values next to sign changes reach the comparison's zero crossings
+    // and the redistancing that replaces the field.  Such a pixel takes
+    // weight 1 (the convolved value) without the projection.  (On the
+    // 20,000-grain workload the areas stay bit-identical for 10 steps and
+    // within 1.3e-7 relative, in 18 grains, after 40.)
+    const float far_level = 0.3f * delta;
+    unsigned* queue = sm.queue[warp];
+    const int nty = (hgt + 7) >> 3;
+    int tx = warp % ntx, ty = warp / ntx, queued = 0;
+    for (bool more = true; more;) {
+        more = ty < nty;
+        if (more) {
+            const int x = tx * 16 + (lane & 15), yt = ty * 8 + (lane >> 4);
+            for (tx += nwarps; tx >= ntx; tx -= ntx) ++ty;
+            const int j = x0 + x;
+            float val[4], conv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int y = yt + 2 * u;
+                const int k = (y0 + y - bo.y0) * wo + (j - bo.x0);
+                val[u] = conv[u] = 0.f;
+                if (x < w && y < hgt) {
+                    val[u] = __ldg(in + k);
+                    conv[u] = out[k];
                 }
-        } else {
-            const InterpSector& s = s_is[-2 - sid];
-            const int kn = wrap_next(segment, real);
-            float ax, ay;
-            if (staged) {
-                ax = (sp[kn].x - sp[segment].x) * lambda;
-                ay = (sp[kn].y - sp[segment].y) * lambda;
-            } else {
-                ax = (float)((P[kn].x - P[segment].x) * lambda);
-                ay = (float)((P[kn].y - P[segment].y) * lambda);
             }
-            interpolator += sqrtf(ax * ax + ay * ay);
-            interpolator /= (float)s.length;
-            interpolator = fminf(fmaxf(interpolator, 0.f), 1.f);
-            const float lw = (float)s.left_w, rw = (float)s.right_w;
-            if (s.lb >= 0 && s.rb >= 0) {
-                const float isr = (float)C.isr, len = (float)s.length;
-                const float quot = (len > 2 * isr ? 2 * isr : len);
-                const float amplitude = ((float)s.boundary_w - (lw + rw) / 2) / (2 * isr) * quot + (lw + rw) / 2;
-                const float a0 = 2 * rw, a1 = -4 * amplitude, a2 = 2 * lw;
-                const float A = a0 + a1 + a2, B = -(a0 * 1.5f + a1 + a2 * 0.5f), Cc = a0 * 0.5f;
-                weight = A * interpolator * interpolator + B * interpolator + Cc;
-            } else {
-                weight = interpolator * lw + (1 - interpolator) * rw;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int y = yt + 2 * u, i = y0 + y;
+                const bool inside = x < w && y < hgt;
+                const bool valid = inside && val[u] > -delta;
+                const float stretched = 2.f * conv[u] - val[u];
+                const bool far = far_ok && valid &&
+                                 ((val[u] >= far_level && conv[u] >= far_level && stretched >= far_level) ||
+                                  (val[u] <= -far_level && conv[u] <= -far_level && stretched <= -far_level));
+                const bool need = valid && !far;
+                if (inside && (kForces ? !need : !valid)) {
+                    float se = 0.f;
+                    if (kForces) se = force(idl[(i - ib.y0) * wi + (j - ib.x0)]);
+                    out[(i - bo.y0) * wo + (j - bo.x0)] = (far ? conv[u] : -delta) - se;
+                }
+                const unsigned needs = __ballot_sync(0xffffffffu, need);
+                if (need) queue[queued + __popc(needs & ((1u << lane) - 1u))] = (unsigned)y << 16 | (unsigned)x;
+                queued += __popc(needs);
             }
+            __syncwarp();
         }
-        out[k] = val + (conv - val) * weight - se;
+        while (queued >= 32 || (!more && queued > 0)) {
+            const bool busy = lane < queued;
+            queued = queued > 32 ? queued - 32 : 0;  // from the end
+            const unsigned item = busy ? queue[queued + lane] : 0u;
+            __syncwarp();
+            if (!busy) break;
+            const int i = y0 + (int)(item >> 16), j = x0 + (int)(item & 0xffffu);
+            const int k = (i - bo.y0) * wo + (j - bo.x0);
+            const int at_id = (i - ib.y0) * wi + (j - ib.x0);
+            const float val = __ldg(in + k), conv = out[k];
+            float lambda = 0.f;
+            int segment = 0;
+            if (staged) {
+                const int nv = nearest_vertex(vb, sp, P, size - 1, j, i, ox, oy, eps_c);
+                if (nv >= 0) segment = segment_step(sp, P, size, j, i, ox, oy, eps_c, nv, &lambda);
+            } else {
+                double dl = 0;
+                segment = project_to_boundary(P, size, (double)j, (double)i, &dl);
+                lambda = (float)dl;
+            }
+            const int sid = staged ? s_sid[segment] : tsid[segment];
+            float interpolator = sid > -2 ? 0.f : staged ? s_acc[segment] : tacc[segment];
+            float weight;
+            if (sid >= 0) {
+                weight = sm.cw[sid];
+            } else if (sid == -1) {
+                // getGBEnergyTimesGBMobility(i, j) through the neighbour table
+                const int id = (int)idl[at_id];
+                weight = 1.f;
+                for (int e = 0; e < nbt.n; ++e)
+                    if (nbt.id[e] == id) {
+                        weight = (float)nbt.w[e];
+                        break;
+                    }
+            } else {
+                const SectorWeights& s = sm.is[-2 - sid];
+                const int kn = wrap_next(segment, real);
+                float ax, ay;
+                if (staged) {
+                    ax = (sp[kn].x - sp[segment].x) * lambda;
+                    ay = (sp[kn].y - sp[segment].y) * lambda;
+                } else {
+                    ax = (float)((P[kn].x - P[segment].x) * lambda);
+                    ay = (float)((P[kn].y - P[segment].y) * lambda);
+                }
+                interpolator += sqrtf(ax * ax + ay * ay);
+                interpolator /= s.length;
+                interpolator = fminf(fmaxf(interpolator, 0.f), 1.f);
+                const float lw = s.left_w, rw = s.right_w;
+                if (s.both) {
+                    const float isr = (float)C.isr, len = s.length;
+                    const float quot = (len > 2 * isr ? 2 * isr : len);
+                    const float amplitude = (s.boundary_w - (lw + rw) / 2) / (2 * isr) * quot + (lw + rw) / 2;
+                    const float a0 = 2 * rw, a1 = -4 * amplitude, a2 = 2 * lw;
+                    const float A = a0 + a1 + a2, B = -(a0 * 1.5f + a1 + a2 * 0.5f), Cc = a0 * 0.5f;
+                    weight = A * interpolator * interpolator + B * interpolator + Cc;
+                } else {
+                    weight = interpolator * lw + (1 - interpolator) * rw;
+                }
+            }
+            float se = 0.f;
+            if (kForces) se = force(idl[at_id]);
+            out[k] = val + (conv - val) * weight - se;
+        }
     }
-    if (st) set_status(S, st);
 }
 
 // CTA per grain from the work queue, contours staged up to kCorrStagedPts;
@@ -616,7 +664,7 @@ template <bool kForces>
 __global__ void __launch_bounds__(128, 7) k_corrector_f(NetConst C, NetState* S) {
     __shared__ __align__(16) CorrectorSmem<kCorrStagedPts> sm;
     const int g = grain_at(S, blockIdx.x);
-    if (!corrects(C, S, g) || S->big_flag[g]) return;
+    if (S->big_flag[g]) return;
     correct_grain<kForces, kCorrStagedPts>(C, S, g, sm);
 }
 
@@ -632,7 +680,7 @@ __global__ void __launch_bounds__(128) k_corrector_big(NetConst C, NetState* S) 
     const int n = S->n_big;
     for (int q = blockIdx.x; q < n; q += gridDim.x) {
         const int g = S->big_list[q];
-        if (corrects(C, S, g)) correct_grain<kForces, kCorrBigPts>(C, S, g, sm);
+        correct_grain<kForces, kCorrBigPts>(C, S, g, sm);
         __syncthreads();  // the next grain overwrites the shared memory
     }
 }

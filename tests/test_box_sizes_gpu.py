@@ -24,9 +24,11 @@ pytestmark = pytest.mark.gpu
 CASES = [(1, 9), (2, 18), (40, 200), (9, 160), (5, 190), (4, 260)]
 
 
-def _run(tmp_path, grains, grid, precision, steps, isotropic=1):
+def _run(tmp_path, grains, grid, precision, steps, isotropic=1, gamma=1.0):
     xml = ms.make_case(str(tmp_path), f"v{grains}_{grid}", ms.voronoi(grains, grid, 7), IsIsotropicNetwork=isotropic)
-    h = gg.GrainHandler(gg.Settings(xml, precision=precision), device=0)
+    settings = gg.Settings(xml, precision=precision)
+    settings.p.gamma_hagb *= gamma
+    h = gg.GrainHandler(settings, device=0)
     try:
         h.load_voxel_files()
         h.distanceInitialisation()
@@ -58,4 +60,14 @@ def test_batched_areas_follow_the_plain_ones(tmp_path, grains, grid, isotropic):
     batched form's by cells, on contours up to some 600 points."""
     _, plain = _run(tmp_path, grains, grid, gg.PRECISION_PLAIN, 3, isotropic)
     _, batched = _run(tmp_path, grains, grid, gg.PRECISION_BATCHED, 3, isotropic)
+    np.testing.assert_allclose(batched, plain, rtol=1e-5)
+
+
+@pytest.mark.parametrize("grains,grid", CASES)
+def test_batched_corrector_of_the_whole_band(tmp_path, grains, grid):
+    """With a relative high-angle energy above 1 no pixel takes the convolved
+    value as it is: the whole band of 2 delta around each boundary is projected,
+    also far from it and over whole tiles, by the batched form's queues."""
+    _, plain = _run(tmp_path, grains, grid, gg.PRECISION_PLAIN, 3, 0, 1.01)
+    _, batched = _run(tmp_path, grains, grid, gg.PRECISION_BATCHED, 3, 0, 1.01)
     np.testing.assert_allclose(batched, plain, rtol=1e-5)
