@@ -21,7 +21,7 @@ constexpr int kSegShared = 512;  // contours up to this length keep their segmen
 struct ConstSector {
     int left, right;  // contour point IDs (-1, -1: whole contour)
     int nj;
-    int js[kMaxSectorJunctions];
+    int8_t js[kMaxSectorJunctions];  // below 64, as many as a grain's junctions
     double weight;
 };
 
@@ -365,14 +365,14 @@ __device__ void build_sectors_warp(const NetConst& C, const NbTable& T, const CP
             }
             ConstSector& c = S.cs[S.nconst];
             c.nj = 1;
-            c.js[0] = jidx;
+            c.js[0] = (int8_t)jidx;
             c.left = jl[jidx];
             c.right = jr[jidx];
             return S.nconst++;
         };
         auto merge = [&](ConstSector& c, int jidx) {
             if (c.nj < kMaxSectorJunctions)
-                c.js[c.nj++] = jidx;
+                c.js[c.nj++] = (int8_t)jidx;
             else
                 st |= S_JUNCTION_OVERFLOW;
         };
@@ -410,7 +410,7 @@ __device__ void build_sectors_warp(const NetConst& C, const NbTable& T, const CP
     // 3. constant-sector weights: mean of junction weights in list order
     for (int s = lane; s < nconst; s += 32) {
         double w = 0;
-        for (int q = 0; q < S.cs[s].nj; ++q) w += jw[S.cs[s].js[q] < 64 ? S.cs[s].js[q] : 63];
+        for (int q = 0; q < S.cs[s].nj; ++q) w += jw[S.cs[s].js[q]];
         S.cs[s].weight = w / (double)S.cs[s].nj;
     }
     __syncwarp();
@@ -681,8 +681,11 @@ __device__ void prepare_sectors_view(const NetConst& C, NetState* S, int g, cons
 // ones at the end of the step; else from the previous roles (after
 // initialisation, grid coarsening or new neighbour lists).
 // A: the type of the per-segment arc lengths (segacc of the form).
+// Serial walks on a few lanes bound it, so as many CTAs per SM as registers
+// and shared memory allow: 20,000 grains 240 us at 20 (88 registers), 202 at 28
+// (206 at 32, which spills more).
 template <bool kCur, typename A>
-__global__ void __launch_bounds__(32) k_sectors(NetConst C, NetState* S) {
+__global__ void __launch_bounds__(32, 28) k_sectors(NetConst C, NetState* S) {
     const int g = grain_at(S, blockIdx.x);
     if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
     __shared__ SectorSet sec;

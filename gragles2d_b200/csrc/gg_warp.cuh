@@ -966,14 +966,19 @@ struct PointInfo {
     double len;
 };
 
-constexpr int kNbPts = 512;  // per-warp shared buffers of the neighbour build
+constexpr int kNbPts = 256;  // per-warp shared buffers of the neighbour build
 
 // LSbox::computeVolumeAndEnergy + ExplicitGrainBoundary::buildDirectNeighbours
 // (src/box.cpp:1201-1228, src/grainBoundary.cpp:85-199), one warp per grain:
 // lanes probe contour points, evaluate the per-pair physics and the terms of
 // the area and energy sums into shared memory; lane 0 builds the neighbour
 // list and adds the terms in contour order (the reference's order; the
-// batched form sums by trees instead).
+// batched form sums by trees instead).  Latency bounds it (a chain of five
+// dependent loads per point, then the FP64 physics of a few neighbours):
+// 20,000 grains 176 us with a point's chain at a time per lane in three passes
+// over the contour, 136 us in one pass with two points' chains side by side (one:
+// 139, four: 144 at 72 registers) and room for 256 points per warp in shared
+// memory, which 99% of a network's contours need at most.
 template <typename R>
 __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst C, NetState* S, PointInfo* scratch) {
     __shared__ int s_cid[kGrainsPerBlock][kNbPts];
@@ -996,50 +1001,77 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst 
     const bool sh = n - 1 <= kNbPts;
     auto CID = [&](int q) -> int& { return sh ? s_cid[wid][q] : info[q].cid; };
     auto LEN = [&](int q) -> double& { return sh ? s_len[wid][q] : info[q].len; };
-    // area (computeVolume, src/grainBoundary.cpp:201-213): terms side by side,
-    // added in contour order (plain) or by a tree (batched, as the sums below)
+    // One pass over the points, kU per lane with each level of their loads in
+    // flight together: the area's terms (computeVolume, src/grainBoundary.cpp:
+    // 201-213; added in contour order in the plain form, by a tree in the
+    // batched one, as the sums below), the segments' lengths, and the probes,
+    // the first failing one of which ends the reference's loop.
     constexpr bool kTree = sizeof(R) == sizeof(float);
+    constexpr int kU = 2;
     double v = 0;
-    if constexpr (kTree) {
-        for (int i = lane; i < n - 1; i += 32) v += (P[i].y + P[i + 1].y) * (P[i].x - P[i + 1].x);
-        v = warp_sum_to_all(v);
-    } else {
-        for (int i0 = 0; i0 < n - 1; i0 += 32) {
-            const int i = i0 + lane;
-            double t = 0;
-            if (i < n - 1) t = (P[i].y + P[i + 1].y) * (P[i].x - P[i + 1].x);
-            const int m = n - 1 - i0 < 32 ? n - 1 - i0 : 32;
-            for (int q = 0; q < m; ++q) v += __shfl_sync(FULL, t, q);
-        }
-    }
-    const double newVolume = fabs(fabs(v) * h * h * 0.5);
-    // probes; the first failing point ends the reference's loop
     int first_bad = 0x7fffffff;
-    for (int i = lane; i < n - 1; i += 32) {
-        const double px = P[i].x, py = P[i].y;
-        int pxGrid = (int)px, pyGrid = (int)py;
-        uint32_t k;
-        bool bad = false;
-        if (!buf_index(bc, pyGrid, pxGrid, &k)) bad = true;
-        if (!bad && (double)phi[k] > 0) {
-            pxGrid = (int)(px + 1);
-            if (!buf_index(bc, pyGrid, pxGrid, &k)) bad = true;
-            if (!bad && (double)phi[k] > 0) {
-                pyGrid = (int)(py + 1);
-                if (!buf_index(bc, pyGrid, pxGrid, &k)) bad = true;
-                if (!bad && (double)phi[k] > 0) pxGrid = (int)px;
+    for (int i0 = 0; i0 < n - 1; i0 += 32 * kU) {
+        double px[kU], py[kU], area[kU], len[kU];
+        uint32_t k[kU], cid[kU];
+        bool bad[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int i = i0 + 32 * u + lane;
+            px[u] = py[u] = area[u] = len[u] = 0;
+            if (i < n - 1) {
+                px[u] = P[i].x;
+                py[u] = P[i].y;
+                const double qx = P[i + 1].x, qy = P[i + 1].y;
+                area[u] = (py[u] + qy) * (px[u] - qx);
+                const double dx = px[u] - qx, dy = py[u] - qy;
+                len[u] = sqrt(dx * dx + dy * dy);
             }
         }
-        if (!bad && (pyGrid < 0 || pyGrid >= bc.y1 || pxGrid < 0 || pxGrid >= bc.x1)) bad = true;
-        if (!bad && !buf_index(bc, pyGrid, pxGrid, &k)) bad = true;
-        uint32_t cid = 0;
-        if (!bad) {
-            cid = idl[k];
-            if (cid != 0 && (cid > (uint32_t)C.N || C.state[cid] == G_GONE)) bad = true;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            // the corners in the reference's order; the first whose field is
+            // not positive is the probe, else the fourth, and a corner outside
+            // the box before that is a failure
+            const int gx = (int)px[u], gy = (int)py[u];
+            const int gx1 = (int)(px[u] + 1), gy1 = (int)(py[u] + 1);
+            uint32_t k0 = 0, k1 = 0, k2 = 0;
+            const bool in0 = buf_index(bc, gy, gx, &k0), in1 = buf_index(bc, gy, gx1, &k1);
+            const bool in2 = buf_index(bc, gy1, gx1, &k2);
+            const bool live = i0 + 32 * u + lane < n - 1;
+            const double f0 = live && in0 ? (double)phi[k0] : 0, f1 = live && in1 ? (double)phi[k1] : 0;
+            const double f2 = live && in2 ? (double)phi[k2] : 0;
+            const bool past0 = in0 && f0 > 0, past1 = past0 && in1 && f1 > 0, past2 = past1 && in2 && f2 > 0;
+            const int x = past0 && !past2 ? gx1 : gx, y = past1 ? gy1 : gy;
+            bad[u] = !in0 || (past0 && !in1) || (past1 && !in2) || y < 0 || y >= bc.y1 || x < 0 || x >= bc.x1;
+            bad[u] = !buf_index(bc, y, x, &k[u]) || bad[u];
         }
-        CID(i) = bad ? -1 : (int)cid;
-        if (bad) first_bad = min(first_bad, i);
+#pragma unroll
+        for (int u = 0; u < kU; ++u) cid[u] = !bad[u] && i0 + 32 * u + lane < n - 1 ? idl[k[u]] : 0u;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (cid[u] > (uint32_t)C.N)
+                bad[u] = true;
+            else if (cid[u] != 0 && C.state[cid[u]] == G_GONE)
+                bad[u] = true;
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int i = i0 + 32 * u + lane;
+            if (i < n - 1) {
+                CID(i) = bad[u] ? -1 : (int)cid[u];
+                LEN(i) = len[u];
+                if (bad[u]) first_bad = min(first_bad, i);
+            }
+            if constexpr (kTree) {
+                v += area[u];
+            } else {
+                const int m = min(n - 1 - (i0 + 32 * u), 32);
+                for (int q = 0; q < m; ++q) v += __shfl_sync(FULL, area[u], q);
+            }
+        }
     }
+    if constexpr (kTree) v = warp_sum_to_all(v);
+    const double newVolume = fabs(fabs(v) * h * h * 0.5);
     first_bad = warp_min_i(first_bad);
     const int upto = first_bad < n - 1 ? first_bad : n - 1;
     __syncwarp();
@@ -1084,8 +1116,7 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst 
         const int i = i0 + lane;
         double term = 0;
         if (i < n - 1) {
-            const double dx = P[i].x - P[i + 1].x, dy = P[i].y - P[i + 1].y;
-            const double len = sqrt(dx * dx + dy * dy);
+            const double len = LEN(i);
             double energy = -1.0;  // generatePoint's value, kept where the loop never reached
             if (i < upto) {
                 // the neighbour's physics, evaluated once per neighbour above
@@ -1104,7 +1135,6 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst 
                 }
                 P[i].mob = mob;
                 P[i].energy = energy;
-                LEN(i) = len * h;
             }
             term = len * energy * h;
         }
@@ -1124,7 +1154,7 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst 
             const int cid = s_nid[wid][e];
             double len = 0;
             for (int i = lane; i < upto; i += 32)
-                if (CID(i) == cid) len += LEN(i);
+                if (CID(i) == cid) len += LEN(i) * h;
             len = warp_sum_to_all(len);
             if (lane == 0) s_nlen[wid][e] = len;
         }
@@ -1137,7 +1167,7 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst 
             len = s_nlen[wid][e];
         } else {
             for (int i = 0; i < upto; ++i)
-                if (CID(i) == cid) len += LEN(i);
+                if (CID(i) == cid) len += LEN(i) * h;
         }
         nb[e].id = cid;
         nb[e].length = len;
