@@ -13,10 +13,11 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
 from gragles2d_b200 import dumpfile, gg
 from gragles2d_b200 import microstructure as ms
-from test_oracle_port import _restate_step
+from test_oracle_port import _restate_step, port
 
 pytestmark = pytest.mark.gpu
 
@@ -24,8 +25,9 @@ pytestmark = pytest.mark.gpu
 CASES = [(1, 9), (2, 18), (40, 200), (9, 160), (5, 190), (4, 260)]
 
 
-def _run(tmp_path, grains, grid, precision, steps, isotropic=1, gamma=1.0):
-    xml = ms.make_case(str(tmp_path), f"v{grains}_{grid}", ms.voronoi(grains, grid, 7), IsIsotropicNetwork=isotropic)
+def _run(tmp_path, grains, grid, precision, steps, isotropic=1, gamma=1.0, micro=None):
+    xml = ms.make_case(str(tmp_path), f"v{grains}_{grid}", micro or ms.voronoi(grains, grid, 7),
+                       IsIsotropicNetwork=isotropic)
     settings = gg.Settings(xml, precision=precision)
     settings.p.gamma_hagb *= gamma
     h = gg.GrainHandler(settings, device=0)
@@ -71,3 +73,61 @@ def test_batched_corrector_of_the_whole_band(tmp_path, grains, grid):
     _, plain = _run(tmp_path, grains, grid, gg.PRECISION_PLAIN, 3, 0, 1.01)
     _, batched = _run(tmp_path, grains, grid, gg.PRECISION_BATCHED, 3, 0, 1.01)
     np.testing.assert_allclose(batched, plain, rtol=1e-5)
+
+
+def _shapes(name, nn):
+    """Labels of grains whose contours are no single ring met by every row twice."""
+    y, x = np.mgrid[0:nn, 0:nn]
+    if name == "comb":  # two grains with interlocking teeth: one long contour each
+        labels = np.where((x // 12) % 2 == 0, 1, 2)
+        labels[:12], labels[-12:] = 1, 2
+    elif name == "islands":  # a grain with holes, and islands of others in it
+        labels = np.ones((nn, nn), int)
+        labels[:, nn - nn // 4:] = 2
+        labels[10:22, 8:20] = 3
+        labels[30:45, 10:28] = 4
+        labels[34:40, 15:22] = 5
+    else:  # blocks that meet at corners: saddles
+        labels = np.where((x // 8 + y // 8) % 2 == 0, 1, 2 + (x // 8) % 2)
+    return labels
+
+
+@pytest.mark.parametrize("name,nn", [("comb", 60), ("comb", 90), ("islands", 60), ("blocks", 48)])
+def test_contours_of_winding_grains(tmp_path, name, nn):
+    """The level set walks a contour in pieces from starts in several rows:
+    long contours between two starts, other contours in the box, and saddles
+    must give the reference's points in its order (bit for bit), from the first
+    contours on."""
+    labels = _shapes(name, nn)
+    n = int(labels.max())
+    rng = np.random.Generator(np.random.PCG64(3))
+    euler = ms.quaternion_to_bunge(ms.shoemake_quaternions(rng, n))
+    micro = ms.Microstructure(labels.astype(ms.voronoi(2, 8, 1).labels.dtype), rng.random((n, 2)), euler)
+    d, _ = _run(tmp_path, n, nn, gg.PRECISION_PLAIN, 2, micro=micro)
+    first = d.records[0]
+    for gid, g in first.grains.items():
+        if g.state == 1:
+            assert g.id_box == g.box
+            pts, _ = port.contour(g.phi, g.box, g.idlocal, gid)
+            np.testing.assert_array_equal(pts, g.contour[:, :2], err_msg=f"contour of grain {gid}")
+    checked = sum(_restate_step(d, r0, r1)[0] for r0, r1 in zip(d.records, d.records[1:]))
+    assert checked >= 2
+
+
+@pytest.mark.parametrize("n", [4, 17, 31, 32, 33, 64, 127])
+def test_static_box_convolution_at_the_edges_of_its_kernels(n):
+    """Boxes up to 32 cells take one CTA, larger ones three kernels.  Four direct
+    sums of at most n terms round by 2 n 2^-53 of their largest partial sum each,
+    in all below 1e-12 of the field's maximum at n = 128."""
+    nn, dt = 800, 3.125e-6
+    x = np.random.default_rng(n).standard_normal((n, n))
+    i2 = np.arange(n // 2 + 1)
+    j2 = np.minimum(np.arange(n), n - np.arange(n))
+    g = np.exp(-np.sqrt(2 / np.pi) * (i2[None, :] ** 2 + j2[:, None] ** 2) * 4.0 * dt * nn ** 2 / n ** 2 * np.pi ** 2)
+    ref = np.fft.irfft2(np.fft.rfft2(x) * g, s=(n, n))
+    src = torch.tensor(x, device="cuda")
+    out = torch.full((n, n), float("nan"), dtype=torch.float64, device="cuda")
+    gg.convolve_box_static(src.data_ptr(), out.data_ptr(), n, dt, nn)
+    np.testing.assert_allclose(out.cpu().numpy(), ref, rtol=0, atol=1e-12 * np.abs(x).max())
+    gg.convolve_box_static(src.data_ptr(), src.data_ptr(), n, dt, nn)  # in place
+    assert torch.equal(src, out)
