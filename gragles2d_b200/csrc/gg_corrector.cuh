@@ -681,6 +681,9 @@ __device__ void prepare_sectors_view(const NetConst& C, NetState* S, int g, cons
 // ones at the end of the step; else from the previous roles (after
 // initialisation, grid coarsening or new neighbour lists).
 // A: the type of the per-segment arc lengths (segacc of the form).
+// An isotropic network has no corrector to read the sectors, so they are built
+// only for grains with so many junctions that a list may overflow, which is an
+// error of the network (36 of the 67 us beside redistancing, 1,000 grains).
 // Serial walks on a few lanes bound it, so as many CTAs per SM as registers
 // and shared memory allow: 20,000 grains 240 us at 20 (88 registers), 202 at 28
 // (206 at 32, which spills more).
@@ -697,6 +700,8 @@ __global__ void __launch_bounds__(32, 28) k_sectors(NetConst C, NetState* S) {
     const int64_t coff = kCur ? S->coff_cur[g] : S->coff_prev[g];
     const CPoint* P = (kCur ? S->contCur : S->contPrev) + coff;
     const int size = kCur ? S->cn_cur[g] : S->cn_prev[g];
+    const int nj = min(kCur ? S->jn_cur[g] : S->jn_prev[g], 64);
+    if (C.isotropic && nj <= kMaxSectorJunctions) return;
     SectorPack* pk = reinterpret_cast<SectorPack*>(C.secpack) + g;
     if (size < 2) {
         if (threadIdx.x == 0) {
@@ -712,7 +717,6 @@ __global__ void __launch_bounds__(32, 28) k_sectors(NetConst C, NetState* S) {
     const Box ib = kCur ? S->box_cur[g] : S->box_prev[g];
     const uint32_t* idl = kCur ? S->idCur + S->off_cur[g] : S->idPrev + S->off_prev[g];
     const Junction* J = (kCur ? S->jCur : S->jPrev) + (int64_t)g * C.jmax;
-    const int nj = min(kCur ? S->jn_cur[g] : S->jn_prev[g], 64);
     prepare_sectors_view(C, S, g, P, size, seg, sec, jw, &s_st, &s_per, nbt, jl, jr, ib, idl, J, nj);
     const int nc = sec.nconst, ni = sec.ninterp;
     if (threadIdx.x == 0) {
