@@ -1115,7 +1115,10 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst 
                 px[u] = P[i].x;
                 py[u] = P[i].y;
                 const double qx = P[i + 1].x, qy = P[i + 1].y;
-                area[u] = (py[u] + qy) * (px[u] - qx);
+                if constexpr (kTree)
+                    v += (py[u] + qy) * (px[u] - qx);
+                else
+                    area[u] = (py[u] + qy) * (px[u] - qx);
                 const double dx = px[u] - qx, dy = py[u] - qy;
                 len[u] = sqrt(dx * dx + dy * dy);
             }
@@ -1155,9 +1158,7 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock) k_neighbours_w(NetConst 
                 LEN(i) = len[u];
                 if (bad[u]) first_bad = min(first_bad, i);
             }
-            if constexpr (kTree) {
-                v += area[u];
-            } else {
+            if constexpr (!kTree) {
                 const int m = min(n - 1 - (i0 + 32 * u), 32);
                 for (int q = 0; q < m; ++q) v += __shfl_sync(FULL, area[u], q);
             }
