@@ -311,7 +311,7 @@ def run_ours(args, rank, world, local_rank):
     dom_bytes = ab.get(dom, 0)
     achieved = dom_bytes / (stage_ms[dom] / 1e3) / 1e9 if dom_bytes else None
     kernel_names = {"convolution": "k_conv_sep", "corrector": "k_corrector_f", "comparison": "k_compare",
-                    "level_set": "k_levelset_w", "redistancing": "k_redistance_s",
+                    "level_set": "k_levelset_w", "redistancing": "k_redistance",
                     "volume_energy_neighbours": "k_neighbours_w + k_sectors"}
     out = {
         "metric": METRIC,
