@@ -970,26 +970,29 @@ __global__ void __launch_bounds__(32 * kGrainsPerBlock, 5) k_levelset_w(NetConst
     const int slot = blockIdx.x * kGrainsPerBlock + wid;
     const int g = slot < C.N ? grain_at(S, slot) : C.N + 1;
     if (g > C.N || halted(S)) return;
-    if (C.state[g] == G_EXISTS && !walk_fits<SmallWalk>(S->box_cur[g])) return;  // k_levelset_big's
+    if (!walk_fits<SmallWalk>(S->box_cur[g])) return;  // k_levelset_big's
     levelset_grain<R>(C, S, g, s_walk[wid]);
 }
 
-// The existing grains whose boxes do not fit the small buffers: one-warp CTAs
-// over all slots (which the work queue, where there is one, orders by
-// descending edge, so that they end at the first existing grain that fits).
+// The grains whose boxes do not fit the small buffers, whatever their state:
+// the two kernels run side by side or one after the other and both write the
+// state (a vanished grain is deleted in the next step, not in the one it
+// vanished in), so a grain belongs to one of them by its box alone, which
+// neither changes.  One-warp CTAs over all slots, a lane per slot; the slots of
+// one CTA are a grid apart, so that the largest boxes, which come first in the
+// work queue, go to different ones.
 template <typename R>
 __global__ void __launch_bounds__(32) k_levelset_big(NetConst C, NetState* S) {
     __shared__ LargeWalk s_walk;
     if (halted(S)) return;
-    for (int slot = blockIdx.x; slot < C.N; slot += gridDim.x) {
-        const int g = grain_at(S, slot);
-        if (C.state[g] != G_EXISTS) continue;  // keeps its place in the queue
-        if (walk_fits<SmallWalk>(S->box_cur[g])) {
-            if (S->order) return;
-            continue;
+    for (int s0 = blockIdx.x; s0 < C.N; s0 += 32 * gridDim.x) {
+        const int slot = s0 + (int)(threadIdx.x * gridDim.x);
+        const int g = slot < C.N ? grain_at(S, slot) : 0;
+        unsigned mine = __ballot_sync(0xffffffffu, g > 0 && !walk_fits<SmallWalk>(S->box_cur[g]));
+        for (; mine; mine &= mine - 1) {
+            levelset_grain<R>(C, S, __shfl_sync(0xffffffffu, g, __ffs(mine) - 1), s_walk);
+            __syncwarp();
         }
-        levelset_grain<R>(C, S, g, s_walk);
-        __syncwarp();
     }
 }
 
