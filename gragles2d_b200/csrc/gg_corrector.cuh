@@ -691,6 +691,8 @@ template <bool kCur, typename A>
 __global__ void __launch_bounds__(32, 28) k_sectors(NetConst C, NetState* S) {
     const int g = grain_at(S, blockIdx.x);
     if (g > C.N || C.state[g] != G_EXISTS || halted(S)) return;
+    // the plain form's run in the corrector's own step: only for what it corrects
+    if (sizeof(A) == 8 && (C.regular[g] == 0 || S->loop == 0)) return;
     __shared__ SectorSet sec;
     __shared__ double jw[64];
     __shared__ uint32_t s_st;
