@@ -817,14 +817,13 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
                     j.lambda = 0;
                     j.x = lf + 0.5;
                     j.y = tp + 0.5;
-                } else {
-                    o.status |= S_JUNCTION_OVERFLOW;
                 }
             }
             jn += __popc(jb);
         }
     }
     if (__any_sync(0xffffffffu, point_overflow)) return -1;
+    if (jn > o.jcap) o.status |= S_JUNCTION_OVERFLOW;  // on every lane: the caller reads the first one's
     o.jn = jn < o.jcap ? jn : o.jcap;
     __syncwarp();
     // insertPoint's duplicate test: a candidate equal to its predecessor is dropped
