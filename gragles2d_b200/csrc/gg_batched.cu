@@ -230,16 +230,6 @@ size_t conv_sep_smem(int tmax, int edge) {
 // latency at 7 CTAs of 72 registers per SM (6: 676, 8 with spills: 676).
 constexpr int kCorrBigPts = 1024;
 
-// Packed FP32 pairs (sm_100 f32x2 arithmetic).
-__device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(unsigned long long v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-
 // Nearest contour vertex of projectToGrainBondary (src/grainBoundary.cpp:
 // 365-381) through a uniform grid of cells over the previous box: the
 // vertices are bucketed by cell (counting sort in shared memory), and a pixel
@@ -847,10 +837,7 @@ cudaError_t batched_init_polygon(const NetConst& C, NetState* dS, cudaStream_t s
 }
 
 cudaError_t batched_stage_kernel(const NetConst& C, NetState* dS, int which, cudaStream_t s, const LaunchCfg& cfg) {
-    const int gt = cfg.grain_threads;
-    const int gblocks = (C.N + gt - 1) / gt;
     const int wblocks = (C.N + kGrainsPerBlock - 1) / kGrainsPerBlock;
-    (void)gblocks;
     switch (which) {
         case 0: k_conv_sep<<<C.N, 128, conv_sep_smem(C.tmax, C.conv_smem_edge), s>>>(C, dS); break;
         case 1: if (!C.isotropic) launch_corrector_f(C, dS, s); break;
@@ -873,10 +860,7 @@ cudaError_t batched_stage_kernel(const NetConst& C, NetState* dS, int which, cud
 
 cudaError_t batched_stages(const NetConst& C, NetState* dS, int stages, cudaStream_t s, const LaunchCfg& cfg) {
     if (C.N <= 0) return cudaSuccess;
-    const int gt = cfg.grain_threads;
-    const int gblocks = (C.N + gt - 1) / gt;
     const int wblocks = (C.N + kGrainsPerBlock - 1) / kGrainsPerBlock;
-    (void)gblocks;
     if (stages & ST_CONV) {
         k_conv_sep<<<C.N, 128, conv_sep_smem(C.tmax, C.conv_smem_edge), s>>>(C, dS);
         if (!C.isotropic) launch_corrector_f(C, dS, s);

@@ -53,14 +53,6 @@ __device__ __forceinline__ const Neighbour* find_characteristic(const NetConst& 
     return nullptr;
 }
 
-// LSbox::getGBEnergyTimesGBMobility(LSbox*) (src/box.cpp:554-561)
-__device__ __forceinline__ double gb_weight_for(const NetConst& C, int owner, int id) {
-    const Neighbour* c = find_characteristic(C, owner, id);
-    const double e = c ? c->energy : 1.0, mo = c ? c->mobility : 1.0;
-    if (e * mo > 0.01) return e * mo;
-    return 0.01;
-}
-
 // The owner's direct-neighbour weights (energy x mobility floored at 0.01)
 // for the per-pixel default weight; entries of removed grains are dropped
 // because a removed grain matches no characteristic.
@@ -215,11 +207,6 @@ __device__ void junction_weights(const NetConst& C, const Junction* J, int nj, i
             }
         }
     }
-}
-
-__device__ __forceinline__ double seg_len(const CPoint* P, int a, int b) {
-    const double dx = P[a].x - P[b].x, dy = P[a].y - P[b].y;
-    return sqrt(dx * dx + dy * dy);
 }
 
 // ContourSector::isSegmentWithinSector (src/contourSector.cpp:184-198)

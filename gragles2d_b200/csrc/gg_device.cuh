@@ -63,10 +63,6 @@ GG_HD bool buf_index(const Box& b, int row, int col, uint32_t* idx) {
     return (int64_t)k < size;
 }
 
-GG_HD bool box_contains(const Box& b, int row, int col) {
-    return row >= b.y0 && row < b.y1 && col >= b.x0 && col < b.x1;
-}
-
 template <typename T>
 GG_HD int sgn(T v) {  // src/utilities.h:27-30
     return (T(0) < v) - (v < T(0));

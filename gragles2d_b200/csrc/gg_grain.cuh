@@ -23,14 +23,6 @@ template <typename R>
 struct Field {
     const R* v;  // row-major values of box b
     Box b;
-    // isInside (src/marchingSquares.cpp:189-196)
-    __device__ __forceinline__ bool inside(int row, int col) const {
-        if (row < b.y0 || row >= b.y1 || col < b.x0 || col >= b.x1) return false;
-        return (double)v[(row - b.y0) * (b.x1 - b.x0) + (col - b.x0)] >= 0;
-    }
-    __device__ __forceinline__ double at(int row, int col) const {
-        return (double)v[(row - b.y0) * (b.x1 - b.x0) + (col - b.x0)];
-    }
 };
 
 struct ContourOut {
@@ -42,70 +34,6 @@ struct ContourOut {
     int jn;
     uint32_t status;
 };
-
-__device__ __forceinline__ void ms_insert(ContourOut& o, double x, double y) {
-    // insertPoint (src/marchingSquares.cpp:197-203)
-    if (o.n == 0 || x != o.pts[o.n - 1].x || y != o.pts[o.n - 1].y) {
-        if (o.n >= o.cap) {
-            o.status |= S_CONTOUR_OVERFLOW;
-            return;
-        }
-        o.pts[o.n].x = x;
-        o.pts[o.n].y = y;
-        o.pts[o.n].energy = -1.0;  // SPoint result(-1,-1,-1,-1)
-        o.pts[o.n].mob = -1.0;
-        o.n++;
-    }
-}
-
-// generatePoint (src/marchingSquares.cpp:204-265)
-template <typename R>
-__device__ __forceinline__ void ms_point(const Field<R>& f, int dir, int top, int bottom, int left, int right,
-                                         double* px, double* py) {
-    double delta, position;
-    switch (dir) {
-        case MS_LEFT:
-            *px = left;
-            if (top < f.b.y0) {
-                *py = bottom;
-            } else {
-                delta = f.at(bottom, left) - f.at(top, left);
-                position = bottom - f.at(bottom, left) / delta;
-                *py = position;
-            }
-            break;
-        case MS_RIGHT:
-            *px = right;
-            if (bottom >= f.b.y1) {
-                *py = top;
-            } else {
-                delta = f.at(top, right) - f.at(bottom, right);
-                position = top + f.at(top, right) / delta;
-                *py = position;
-            }
-            break;
-        case MS_UP:
-            *py = top;
-            if (right >= f.b.x1) {
-                *px = left;
-            } else {
-                delta = f.at(top, left) - f.at(top, right);
-                position = left + f.at(top, left) / delta;
-                *px = position;
-            }
-            break;
-        default:  // MS_DOWN
-            *py = bottom;
-            if (left < f.b.x0) {
-                *px = right;
-            } else {
-                delta = f.at(bottom, right) - f.at(bottom, left);
-                position = right - f.at(bottom, right) / delta;
-                *px = position;
-            }
-            break;
-    }
-}
 
 __device__ __forceinline__ void insert_distinct(uint32_t v, uint32_t* arr, int& cnt) {
     // insertDistinctInteger (src/marchingSquares.cpp:303-318)
@@ -151,92 +79,6 @@ __device__ __forceinline__ void ms_junction(const Field<R>& f, const uint32_t* i
         j.x = left + 0.5;
         j.y = top + 0.5;
     }
-}
-
-// MarchingSquaresAlgorithm::generateContour (src/marchingSquares.cpp:28-188).
-// Returns false when no pixel of the box has phi >= 0.  The walk is bounded
-// by 4 (w+2)(h+2) + 16 moves (the reference's loop has no bound).
-template <typename R>
-__device__ bool ms_contour(const Field<R>& f, const uint32_t* idl, uint32_t own, ContourOut& o) {
-    o.n = 0;
-    o.jn = 0;
-    int startX = -1, startY = -1;
-    for (int i = f.b.y0; i < f.b.y1 && startX < 0; i++) {
-        for (int j = f.b.x0; j < f.b.x1; j++) {
-            if (f.inside(i, j)) {
-                startX = j;
-                startY = i;
-                break;
-            }
-        }
-    }
-    if (startX == startY && startX == -1) return false;
-
-    int left = startX - 1, right = startX, top = startY - 1, bottom = startY;
-    int next = MS_NONE, prev = MS_NONE;
-    const long limit = 4L * (box_w(f.b) + 2) * (box_h(f.b) + 2) + 16;
-    long it = 0;
-    do {
-        int mask = 0;
-        if (f.inside(top, left)) mask |= C_TL;
-        if (f.inside(top, right)) mask |= C_TR;
-        if (f.inside(bottom, left)) mask |= C_BL;
-        if (f.inside(bottom, right)) mask |= C_BR;
-        bool emit = true;
-        switch (mask) {
-            case C_TL: next = MS_UP; break;
-            case C_TR: next = MS_RIGHT; break;
-            case C_TL | C_TR: next = MS_RIGHT; break;
-            case C_BL: next = MS_LEFT; break;
-            case C_BL | C_TL: next = MS_UP; break;
-            case C_BL | C_TR:
-                next = (prev == MS_UP) ? MS_RIGHT : MS_LEFT;
-                emit = false;
-                break;
-            case C_BL | C_TR | C_TL: next = MS_RIGHT; break;
-            case C_BR: next = MS_DOWN; break;
-            case C_BR | C_TL:
-                next = (prev == MS_RIGHT) ? MS_DOWN : MS_UP;
-                emit = false;
-                break;
-            case C_BR | C_TR: next = MS_DOWN; break;
-            case C_BR | C_TR | C_TL: next = MS_DOWN; break;
-            case C_BR | C_BL: next = MS_LEFT; break;
-            case C_BR | C_BL | C_TL: next = MS_UP; break;
-            case C_BR | C_BL | C_TR: next = MS_LEFT; break;
-            default: emit = false; break;  // 0 or 15: direction unchanged
-        }
-        if (emit) {
-            double px, py;
-            ms_point(f, next, top, bottom, left, right, &px, &py);
-            ms_insert(o, px, py);
-        }
-        ms_junction(f, idl, own, mask, top, bottom, left, right, o);
-        switch (next) {
-            case MS_UP: top--; bottom--; break;
-            case MS_DOWN: top++; bottom++; break;
-            case MS_LEFT: left--; right--; break;
-            case MS_RIGHT: left++; right++; break;
-            default: break;
-        }
-        prev = next;
-        if (++it > limit) {
-            o.status |= S_WALK_LIMIT;
-            break;
-        }
-    } while (left != startX - 1 || bottom != startY);
-
-    if (o.n > 0) {
-        if (o.pts[0].x != o.pts[o.n - 1].x || o.pts[0].y != o.pts[o.n - 1].y) {
-            if (o.n >= o.cap) {
-                o.status |= S_CONTOUR_OVERFLOW;
-            } else {
-                o.pts[o.n] = o.pts[0];
-                o.n++;
-            }
-        }
-    }
-    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -328,20 +170,6 @@ __device__ int project_to_boundary(const CPoint* P, int asize, double px, double
     return segment_of_vertex(P, asize, px, py, nearest, out_lambda);
 }
 
-// Junction projection of extractBoundaryAndJunctions (src/grainBoundary.cpp:51-61)
-__device__ void project_junctions(const CPoint* P, int n, Junction* js, int jn) {
-    if (n < 2) return;
-    double lambda = 0.0;  // one variable for all junctions, as in the reference
-    for (int i = 0; i < jn; ++i) {
-        int seg = project_to_boundary(P, n, js[i].x, js[i].y, &lambda);
-        const int nx = periodic(seg + 1, n);
-        js[i].x = P[seg].x + (P[nx].x - P[seg].x) * lambda;
-        js[i].y = P[seg].y + (P[nx].y - P[seg].y) * lambda;
-        js[i].segment = seg;
-        js[i].lambda = lambda;
-    }
-}
-
 // computeVolume (src/grainBoundary.cpp:201-213)
 __device__ __forceinline__ double contour_volume(const CPoint* P, int n, double h) {
     double v = 0;
@@ -357,16 +185,6 @@ __device__ __forceinline__ double contour_perimeter(const CPoint* P, int n, doub
         p += sqrt(dx * dx + dy * dy) * h;
     }
     return p;
-}
-
-// computeEnergy (src/grainBoundary.cpp:215-222)
-__device__ __forceinline__ double contour_energy(const CPoint* P, int n, double h) {
-    double e = 0;
-    for (int i = 0; i < n - 1; i++) {
-        const double dx = P[i].x - P[i + 1].x, dy = P[i].y - P[i + 1].y;
-        e += sqrt(dx * dx + dy * dy) * P[i].energy * h;
-    }
-    return e;
 }
 
 // LSbox::isMotionRegular (src/box.cpp:1155-1190); *flag_irregular is set in

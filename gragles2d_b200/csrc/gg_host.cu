@@ -177,7 +177,7 @@ struct gg_ctx {
     bool stats_wanted = false;
     bool stats_fresh = false;
     uint32_t* h_status = nullptr;
-    LaunchCfg cfg{256, 64, {nullptr, nullptr}, nullptr};
+    LaunchCfg cfg{256, {nullptr, nullptr}, nullptr};
 
     cudaGraphExec_t graph = nullptr;
     bool sectors_stale = false;    // batched form: the corrector's sectors need a rebuild before the next step

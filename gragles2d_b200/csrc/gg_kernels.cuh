@@ -21,54 +21,8 @@ __device__ __forceinline__ R* phiB_of(NetState* S) {
     return reinterpret_cast<R*>(S->phiB);
 }
 
-// ---------------------------------------------------------------------------
-// LSbox::computeSecondOrderNeighbours (src/box.cpp:1027-1068): one thread per
-// grain.  New list = existing members of the previous list, in order, then
-// members of their lists whose (convolution) boxes intersect ours, first
-// occurrence only, excluding ourselves.
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ bool boxes_intersect(const Box& a, const Box& b) {  // checkIntersection, src/box.cpp:881-888
     return !(a.x0 > b.x1 || a.x1 < b.x0 || a.y0 > b.y1 || a.y1 < b.y0);
-}
-
-__global__ void k_second_order(NetConst C, NetState* S) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (g > C.N || C.state[g] != G_EXISTS) return;
-    const int K = C.kmax;
-    const int* sec = C.sec_ids + (int64_t)g * K;
-    const int ns = C.sec_n[g];
-    int* cmp = C.cmp_ids + (int64_t)g * K;
-    int nc = 0;
-    bool overflow = false;
-    for (int a = 0; a < ns; ++a) {
-        const int id = sec[a];
-        if (C.state[id] == G_EXISTS) {
-            if (nc < K) cmp[nc++] = id; else overflow = true;
-        }
-    }
-    const Box mine = S->box_cur[g];
-    for (int a = 0; a < ns; ++a) {
-        const int id = sec[a];
-        const int* s2 = C.sec_ids + (int64_t)id * K;
-        const int n2 = C.sec_n[id];
-        for (int q = 0; q < n2; ++q) {
-            const int c = s2[q];
-            if (C.state[c] != G_EXISTS) continue;
-            if (!boxes_intersect(mine, S->box_cur[c])) continue;
-            if (c == g || c == 0) continue;
-            bool in = false;
-            for (int e = 0; e < nc; ++e)
-                if (cmp[e] == c) {
-                    in = true;
-                    break;
-                }
-            if (!in) {
-                if (nc < K) cmp[nc++] = c; else overflow = true;
-            }
-        }
-    }
-    C.cmp_n[g] = nc;
-    if (overflow) set_status(S, S_LIST_OVERFLOW);
 }
 
 // ---------------------------------------------------------------------------
@@ -298,15 +252,9 @@ __global__ void __launch_bounds__(256) k_compare(NetConst C, NetState* S) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// grainhdl::level_set -> LSbox::extractContour (src/grainhdl.cpp:830-848,
-// src/box.cpp:1089-1153): one thread per grain.  Removes grains marked as
-// vanished, extracts contour and junctions from the compared field, retries
-// after clearing on irregular motion, and computes the next (square) box.
-// ---------------------------------------------------------------------------
+// LSbox::clearContourGrainArea (src/box.cpp:1888-1906) by one lane.
 template <typename R>
 __device__ bool clear_contour_area(R* phi, const Box& b, const CPoint* P, int n, double h) {
-    // LSbox::clearContourGrainArea (src/box.cpp:1888-1906)
     if (n == 0) return true;
     double minx = P[0].x, maxx = P[0].x, miny = P[0].y, maxy = P[0].y;
     for (int i = 0; i < n; i++) {
@@ -326,72 +274,6 @@ __device__ bool clear_contour_area(R* phi, const Box& b, const CPoint* P, int n,
             if ((double)phi[k] >= 0) phi[k] = (R)(-h);
         }
     return ok;
-}
-
-template <typename R>
-__global__ void k_levelset(NetConst C, NetState* S) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (g > C.N || halted(S)) return;
-    const int st = C.state[g];
-    const Box bc = S->box_cur[g];
-    if (st != G_EXISTS) {
-        if (st == G_VANISHED) {  // delete grains[id] (src/grainhdl.cpp:840-842)
-            C.state[g] = G_GONE;
-            C.gone_loop[g] = S->loop;
-        }
-        S->box_new[g] = bc;
-        S->cn_cur[g] = 0;
-        S->jn_cur[g] = 0;
-        return;
-    }
-    C.regular[g] = 1;
-    const int old_len = S->cn_prev[g];
-    R* phi = phiA_of<R>(S) + S->off_cur[g];
-    Field<R> f{phi, bc};
-    const uint32_t* idl = S->idCur + S->off_cur[g];
-    ContourOut o{S->contCur + S->coff_cur[g], S->ccap_cur[g], 0, S->jCur + (int64_t)g * C.jmax, C.jmax, 0, 0};
-    int irregular = 0;
-    bool ok = ms_contour(f, idl, (uint32_t)g, o);
-    if (ok) {
-        project_junctions(o.pts, o.n, o.js, o.jn);
-        double newVolume = contour_volume(o.pts, o.n, C.h);
-        if (!motion_regular(old_len, o.n, C.volume[g], newVolume, C.dt, &irregular)) {
-            int tries = 0;
-            do {
-                if (!clear_contour_area(phi, bc, o.pts, o.n, C.h)) o.status |= S_INDEX;
-                ok = ms_contour(f, idl, (uint32_t)g, o);
-                if (!ok) break;
-                project_junctions(o.pts, o.n, o.js, o.jn);
-                newVolume = contour_volume(o.pts, o.n, C.h);
-                if (++tries > 64) {
-                    o.status |= S_RETRY_LIMIT;
-                    break;
-                }
-            } while (!motion_regular(old_len, o.n, C.volume[g], newVolume, C.dt, &irregular));
-        }
-    }
-    if (o.status) set_status(S, o.status);
-    if (!ok) {
-        C.state[g] = G_VANISHED;
-        S->box_new[g] = bc;
-        S->cn_cur[g] = 0;
-        S->jn_cur[g] = 0;
-        return;
-    }
-    if (irregular) C.regular[g] = 0;
-    int* nb = C.newbb + 4 * (int64_t)g;
-    Box nbx = bc;
-    if (!C.decouple) {
-        if (nb[0] < 0) nb[0] = 0;
-        if (nb[2] < 0) nb[2] = 0;
-        if (nb[1] > C.m) nb[1] = C.m;
-        if (nb[3] > C.m) nb[3] = C.m;
-        nbx = resize_to_square(Box{nb[0], nb[1], nb[2], nb[3]}, C.m);
-    }
-    S->box_new[g] = nbx;
-    C.perimeter[g] = contour_perimeter(o.pts, o.n, C.h);
-    S->cn_cur[g] = o.n;
-    S->jn_cur[g] = o.jn;
 }
 
 // ---------------------------------------------------------------------------
@@ -517,85 +399,6 @@ __global__ void __launch_bounds__(1024) k_alloc(NetConst C, NetState* S, int spe
         }
     }
     if (range) set_status(S, S_TABLE_RANGE);
-}
-
-// ---------------------------------------------------------------------------
-// LSbox::computeVolumeAndEnergy + ExplicitGrainBoundary::buildDirectNeighbours
-// (src/box.cpp:1201-1228, src/grainBoundary.cpp:85-199): one thread per grain.
-// ---------------------------------------------------------------------------
-template <typename R>
-__global__ void k_neighbours(NetConst C, NetState* S) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int loop = S->loop;
-    if (g > C.N || C.state[g] != G_EXISTS || C.regular[g] == 0 || halted(S)) return;
-    CPoint* P = S->contCur + S->coff_cur[g];
-    const int n = S->cn_cur[g];
-    const double h = C.h;
-    const double newVolume = fabs(contour_volume(P, n, h));
-    const Box bc = S->box_cur[g];
-    const R* phi = phiA_of<R>(S) + S->off_cur[g];
-    const uint32_t* idl = S->idCur + S->off_cur[g];
-    Neighbour* nb = C.nb + (int64_t)g * C.nbmax;
-    int nn = 0;
-    bool invalid = false, overflow = false;
-    const double* qg = C.quat + 4 * (int64_t)g;
-    for (int i = 0; i < n - 1; i++) {
-        const double px = P[i].x, py = P[i].y;
-        int pxGrid = (int)px, pyGrid = (int)py;
-        uint32_t k;
-        if (!buf_index(bc, pyGrid, pxGrid, &k)) { invalid = true; break; }
-        if ((double)phi[k] > 0) {
-            pxGrid = (int)(px + 1);
-            if (!buf_index(bc, pyGrid, pxGrid, &k)) { invalid = true; break; }
-            if ((double)phi[k] > 0) {
-                pyGrid = (int)(py + 1);
-                if (!buf_index(bc, pyGrid, pxGrid, &k)) { invalid = true; break; }
-                if ((double)phi[k] > 0) pxGrid = (int)px;
-            }
-        }
-        // LSbox::getNeighbourAt (src/box.cpp:2190-2195)
-        if (pyGrid < 0 || pyGrid >= bc.y1 || pxGrid < 0 || pxGrid >= bc.x1) { invalid = true; break; }
-        if (!buf_index(bc, pyGrid, pxGrid, &k)) { invalid = true; break; }
-        const uint32_t cid = idl[k];
-        if (cid != 0 && (cid > (uint32_t)C.N || C.state[cid] == G_GONE)) { invalid = true; break; }
-        const double theta = grain_misorientation(qg, C.quat + 4 * (int64_t)cid);
-        P[i].mob = mobility_model(theta, C);
-        P[i].energy = read_shockley(theta, C);
-        const double dx = P[i].x - P[i + 1].x, dy = P[i].y - P[i + 1].y;
-        const double line_length = sqrt(dx * dx + dy * dy) * h;
-        int e = 0;
-        for (; e < nn; ++e)
-            if (nb[e].id == (int)cid) break;
-        if (e == nn) {
-            if (nn >= C.nbmax) {
-                overflow = true;
-                continue;
-            }
-            nb[nn].id = (int)cid;
-            nb[nn].length = 0;
-            nb[nn].energy = P[i].energy;
-            nb[nn].misori = theta;
-            nb[nn].mobility = P[i].mob;
-            nn++;
-        }
-        nb[e].length += line_length;
-    }
-    C.nb_n[g] = nn;
-    if (overflow) set_status(S, S_NEIGHBOUR_OVERFLOW);
-    if (invalid) {
-        C.regular[g] = 0;  // markAsInvalidMotion (src/box.cpp:1939-1945)
-    } else if (n > 0) {
-        P[n - 1].energy = P[0].energy;
-        P[n - 1].mob = P[0].mob;
-    }
-    C.energy[g] = contour_energy(P, n, h);
-    double dA = newVolume - C.volume[g];
-    dA = dA / C.dt;
-    dA = dA * (3 / kPi);
-    const unsigned int lp = (unsigned int)loop;
-    if ((unsigned long)(lp - 1u) % (unsigned long)C.analysis_timestep == 0 || lp == 0) C.meanda[g] = 0;
-    C.meanda[g] += dA;
-    C.volume[g] = newVolume;
 }
 
 // LSbox::resizeGrid (src/box.cpp:1408-1485) of one grain (not removed) per

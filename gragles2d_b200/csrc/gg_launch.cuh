@@ -22,7 +22,6 @@ enum : int {
 
 struct LaunchCfg {
     int compare_threads;
-    int grain_threads;  // one-thread-per-grain kernels
     // further streams and events of the context, for launches that run side by side
     cudaStream_t side[2];
     cudaEvent_t* ev;

@@ -252,10 +252,7 @@ cudaError_t traffic_launch(const NetConst& C, NetState* dS, cudaStream_t s) {
 }
 
 cudaError_t plain_stage_kernel(const NetConst& C, NetState* dS, int which, cudaStream_t s, const LaunchCfg& cfg) {
-    const int gt = cfg.grain_threads;
-    const int gblocks = (C.N + gt - 1) / gt;
     const int wblocks = (C.N + kGrainsPerBlock - 1) / kGrainsPerBlock;
-    (void)gblocks;
     switch (which) {
         case 0: return launch_convolution_plain(C, dS, s, cfg, false, false);
         case 1:
@@ -277,10 +274,7 @@ cudaError_t plain_stage_kernel(const NetConst& C, NetState* dS, int which, cudaS
 
 cudaError_t plain_stages(const NetConst& C, NetState* dS, int stages, cudaStream_t s, const LaunchCfg& cfg) {
     if (C.N <= 0) return cudaSuccess;
-    const int gt = cfg.grain_threads;
-    const int gblocks = (C.N + gt - 1) / gt;
     const int wblocks = (C.N + kGrainsPerBlock - 1) / kGrainsPerBlock;
-    (void)gblocks;
     // tangent mode (C.dvol set): the tangent kernels of gg_tangent.cuh follow
     // their stages; the corrector's tangent reads the uncorrected convolution,
     // so it runs first

@@ -753,7 +753,7 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
                 next[k] = nx;
                 emit[k] = (kMsEmit >> m) & 1u;
                 const int lf = left[k], tp = top[k], right = lf + 1, bottom = tp + 1;
-                // generatePoint's values: a then c, delta = a - c (ms_point)
+                // generatePoint's values: a then c, delta = a - c (src/marchingSquares.cpp:204-265)
                 const int ra = nx == MS_RIGHT || nx == MS_UP ? tp : bottom;
                 const int ca = nx == MS_LEFT || nx == MS_UP ? lf : right;
                 const int rc = nx == MS_LEFT ? tp : nx == MS_RIGHT ? bottom : ra;
@@ -777,7 +777,7 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
         for (int k = 0; k < 2; ++k) {
             const int lf = left[k], tp = top[k], right = lf + 1, bottom = tp + 1;
             double px = 0, py = 0;
-            if (emit[k]) {  // generatePoint (ms_point) on the loaded values
+            if (emit[k]) {  // generatePoint on the loaded values
                 const int nx = next[k];
                 const bool across = nx == MS_LEFT || nx == MS_RIGHT;
                 // from the first value's corner to the second one's
