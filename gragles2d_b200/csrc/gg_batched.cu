@@ -212,8 +212,8 @@ size_t conv_sep_smem(int tmax, int edge) {
     return sizeof(float) * (staged > kernel_only ? staged : kernel_only);
 }
 
-// Batched-form corrector: same sectors as k_corrector (built by one warp),
-// with the previous contour staged in shared memory (FP32 box-local
+// Batched-form corrector: same sectors as k_corrector (from k_sectors), with
+// the previous contour staged in shared memory (FP32 box-local
 // coordinates) and the per-pixel work in FP32, except the discrete decisions
 // of the projection, which follow the reference's FP64 arithmetic.  Each
 // warp scans the box in tiles and collects the pixels near the boundary, about a
@@ -233,8 +233,8 @@ constexpr int kCorrBigPts = 1024;
 // Nearest contour vertex of projectToGrainBondary (src/grainBoundary.cpp:
 // 365-381) through a uniform grid of cells over the previous box: the
 // vertices are bucketed by cell (counting sort in shared memory), and a pixel
-// measures, in FP64 from the contour itself, the vertices of the 3 x 3 cells
-// around its own.  Every vertex within `cell` of the pixel lies in that
+// measures the vertices of the 3 x 3 cells around its own (in FP32, near-ties
+// again in FP64 from the contour itself: see nearest_vertex).  Every vertex within `cell` of the pixel lies in that
 // window, so when the smallest distance found is at most (cell - 1e-3)^2 (the
 // margin covers the cell index of a vertex on a cell edge) it is the smallest
 // over the whole contour; ties go to the lowest index, as the reference's

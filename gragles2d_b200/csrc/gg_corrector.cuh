@@ -1,8 +1,8 @@
 // Anisotropic velocity corrector of the convolution stage
-// (LSbox::executeConvolution, src/box.cpp:428-531): per grain, contour
-// sectors around the previous step's junctions are built by one warp into
-// shared memory, then every pixel projects onto the previous contour and
-// blends its convolved value with the sector / junction / boundary weight.
+// (LSbox::executeConvolution, src/box.cpp:428-531): k_sectors builds, a warp per
+// grain, the contour sectors around the previous step's junctions; in the
+// corrector of either form every pixel then projects onto the previous contour
+// and blends its convolved value with the sector / junction / boundary weight.
 #pragma once
 
 #include <cfloat>
@@ -670,7 +670,9 @@ __device__ void prepare_sectors_view(const NetConst& C, NetState* S, int g, cons
 // A: the type of the per-segment arc lengths (segacc of the form).
 // An isotropic network has no corrector to read the sectors, so they are built
 // only for grains with so many junctions that a list may overflow, which is an
-// error of the network (36 of the 67 us beside redistancing, 1,000 grains).
+// error of the network (36 of the 67 us beside redistancing, 1,000 grains).  So
+// S_INDEX and S_SECTOR_GUARD of the others' sectors are not set there, as the
+// plain form, which builds none, does not set them either.
 // Serial walks on a few lanes bound it, so as many CTAs per SM as registers
 // and shared memory allow: 20,000 grains 240 us at 20 (88 registers), 202 at 28
 // (206 at 32, which spills more).

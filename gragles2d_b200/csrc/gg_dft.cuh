@@ -21,7 +21,7 @@
 //
 // Measured (B200, stage time; before: one output per thread, both spectra and
 // the table in device memory): 5,000 boxes 2.52 -> 0.95 ms, 1,000 boxes of mean
-// edge 44 742 -> 217 us.  The FP64 pipe is then busy half of the time; the rest
+// edge 44 742 -> 220 us.  The FP64 pipe is then busy half of the time; the rest
 // is the loop's own latency and the barriers between the transforms (2, 3 or 4
 // CTAs per SM make no difference).
 #pragma once

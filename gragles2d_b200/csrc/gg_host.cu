@@ -1416,7 +1416,9 @@ int gg_distance_initialisation(gg_ctx* c) {
     // that a box's list loads and its last tiles hide behind more other boxes
     // (us of the stage with 256 / 128 / 64 threads: 60 boxes 21 / 31 / 51, 1,000
     // 33 / 42 / 70, 2,000 64 / 65 / 113, 20,000 591 / 427 / 401, 100,000 clustered
-    // 3,394 / 2,424 / 2,230; FP64 5,000 201 / 196 / 235).
+    // 3,394 / 2,424 / 2,230; FP64 5,000 201 / 196 / 235).  The count is the one at
+    // initialisation: a network of 20,000 grains that has coarsened to 390 keeps
+    // its 64 threads, 54 us of its step's 358.
     c->cfg.compare_threads = N < 2048 ? 256 : (N < 8192 ? 128 : 64);
     C.conv_smem_edge = 64;
     C.isotropic = P.is_isotropic_network ? 1 : 0;

@@ -1,9 +1,10 @@
 // Warp-per-grain versions of the per-grain sequential stages (level set,
 // volume/energy/neighbours, second-order lists).  The parts of each
 // reference routine that are independent per pixel, per contour point or per
-// list entry run across the 32 lanes; every order-dependent part (the
-// marching-squares walk, list construction, sums) runs on lane 0 in the
-// reference's order, so the FP64 form stays bit-identical.
+// list entry run across the 32 lanes; every order-dependent part keeps the
+// reference's order, so the FP64 form stays bit-identical: the marching-squares
+// walk is put together from pieces, and sums add their terms one by one (the
+// batched form's by trees).
 #pragma once
 
 #include "gg_grain.cuh"
@@ -421,7 +422,7 @@ __device__ bool clear_area_xy(R* phi, const Box& b, const double2* P, int n, dou
 
 // Shared buffers of one warp's contour extraction: the padded bitmap of the
 // box, the recorded walk steps, the contour points (before them, the starts and
-// pieces of walk_parallel).  Boxes up to about 94 cells take the small ones, four
+// pieces of walk_parallel).  Boxes up to 97 cells take the small ones, four
 // warps to a CTA; larger ones (to 222 cells) a CTA of one warp with the large
 // ones, beside them.  What fits neither is walked by one lane in device memory,
 // which takes some 250 us for a box of 100 cells.  (Smaller buffers at seven CTAs
@@ -450,8 +451,8 @@ __device__ int extract_bitmap_warp(const Field<R>& f, const uint32_t* idl, uint3
 // Contour + junctions of one grain by one warp; returns false if no pixel
 // has phi >= 0.  The walk writes into the warp's shared buffer xy (or, for a
 // contour longer than the buffer, directly into the global contour);
-// junctions are projected one lane per junction.  On return *in_shared says
-// where the points are.
+// junctions are projected by four lanes each (one where the points are not in
+// shared memory).  On return *in_shared says where the points are.
 template <class W, typename R>
 __device__ bool extract_warp(const Field<R>& f, const uint32_t* idl, uint32_t own, ContourOut& o, int lane, W& ws,
                              bool* in_shared) {

@@ -57,7 +57,9 @@ enum {
     GG_S_NEIGHBOUR_OVERFLOW = 1 << 6,
     GG_S_NAN = 1 << 7,
     GG_S_INDEX = 1 << 8,         /* an access the reference would have faulted on */
-    GG_S_SECTOR_GUARD = 1 << 9,  /* a sector walk met a zero-length contour */
+    GG_S_SECTOR_GUARD = 1 << 9,  /* a sector walk met a zero-length contour (sectors are built for the corrector:
+                                    in isotropic networks this bit, and GG_S_INDEX of a sector, are not set but
+                                    for grains of more than 24 junctions in the batched form) */
     GG_S_RETRY_LIMIT = 1 << 10   /* more than 64 contour re-extractions */
 };
 
